@@ -280,8 +280,8 @@ int titus_limited_flux(int32_t nx, int32_t ny, int32_t q, double dx, double dy, 
  * collision (I + dE D)^{-1}, in-scattering from psi, and the dose with csd.SMid
  * (problem->stopping_mid must be set). It is the r -> N limit the DLR
  * integrators approach. titus_pn_full_solve_device runs the whole sweep on
- * `stream` (a cudaStream_t, NULL = default) as one captured CUDA graph of two
- * kernels per energy step; options->max_steps bounds the steps (0 = all).
+ * `stream` (a cudaStream_t, NULL = default) as one captured CUDA graph of one
+ * kernel per energy step; options->max_steps bounds the steps (0 = all).
  * titus_pn_full_fetch waits and copies u (n x N, raw: the reference returns
  * 1/2 sqrt(gamma_0) u), the dose (n) and psi (n x q) to host buffers (each may
  * be NULL). titus_pn_full_solve does both. */
@@ -324,7 +324,7 @@ int titus_create_3d(const titus_problem_t* problem, const titus_problem_3d_t* ex
  * titus_pn_full_solve's sweep, transposed stencils and P_N products run from
  * the last energy step back to the first; checkpoint_every = k keeps (u, psi)
  * entering every k-th step from one forward pass and recomputes each segment
- * (0 = about sqrt(steps)); device memory about (steps/k + k + 12) n N words.
+ * (0 = about sqrt(steps)); device memory about (steps/k + k + 4) n N words.
  * weight, target, dj_ddose and the outputs are host arrays (NULL weight = 1,
  * NULL target = 0, NULL outputs are skipped). Synchronous. FP64 only. */
 int titus_dose_adjoint(titus_solver_t* solver, int32_t method, const titus_options_t* options, const double* weight,
