@@ -1078,14 +1078,19 @@ static __device__ __noinline__ int w_truncate_svd(WCtx& x, int m) {
     const double tol = x.P.theta * pow(sqrt(nrm), x.P.theta_index);
     const int half = m / 2;
     int kk = half;
-    for (int j = 1; j <= 2 * half; ++j) {
+    // thread j - 1 forms the tail sum from j on; the first one below tol decides
+    __shared__ double s_tail[KA];
+    for (int j = threadIdx.x; j < 2 * half; j += NT) {
         double tail = 0.0;
-        for (int i = j - 1; i < 2 * half; ++i) tail += sm->sig[i];
-        if (fabs(tail) < tol) {
+        for (int i = j; i < 2 * half; ++i) tail += sm->sig[i];
+        s_tail[j] = tail;
+    }
+    __syncthreads();
+    for (int j = 1; j <= 2 * half; ++j)
+        if (fabs(s_tail[j - 1]) < tol) {
             kk = j;
             break;
         }
-    }
     kk = min(kk, x.P.r);
     kk = max(kk, 2);
     kk = min(kk, m);

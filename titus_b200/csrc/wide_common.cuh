@@ -33,7 +33,7 @@ constexpr int NOPS_W = TITUS_WIDE_NOPS;
 constexpr bool kThreeD = NOPS_W == 6;
 static_assert(NOPS_W == 4 || NOPS_W == 6, "four (2D) or six (3D) streaming pairs");
 
-constexpr int NT = titus::NT;   // threads per CTA
+constexpr int NT = 512;   // threads per CTA
 constexpr int RA = titus::WIDE_RA;   // max rank entering a step
 constexpr int KA = 2 * RA;      // max augmented width
 constexpr int LDS = KA + 1;     // row stride of the truncation SVD's column arrays (odd: no bank conflicts)
@@ -186,10 +186,11 @@ __device__ inline bool wreduce(WCtx& x, int count, Hook hook) {
         ProfScope ps(x.prof, PF_REDUCE);
         // CTA b sums the slice [e0, e1) over the G partials. Blocks of RCH
         // elements x RSPL partial-splits keep RSPL independent L2 loads in
-        // flight per element (adjacent threads read adjacent elements); the
-        // splits are combined in a fixed order, so the sum is deterministic.
+        // flight per element (adjacent threads read adjacent elements); a warp
+        // folds its two splits, the rest are combined in a fixed order, so the
+        // sum is deterministic.
         constexpr int RCH = 16, RSPL = NT / RCH;
-        __shared__ double s_part[NT];
+        __shared__ double s_part[NT / 2];
         const int per = (count + x.G - 1) / x.G;
         const int e0 = x.b * per, e1 = min(count, e0 + per);
         const double* base = x.st.part + (size_t)x.parity * x.G * PMAXW;
@@ -200,11 +201,12 @@ __device__ inline bool wreduce(WCtx& x, int count, Hook hook) {
             double a = 0.0;
             if (e < e1)
                 for (int g = sp; g < x.G; g += RSPL) a += ldcg(base + (size_t)g * PMAXW + e);
-            s_part[threadIdx.x] = a;
+            a += __shfl_xor_sync(0xffffffffu, a, RCH);
+            if ((threadIdx.x & 31) < RCH) s_part[threadIdx.x / 32 * RCH + el] = a;
             __syncthreads();
             if (threadIdx.x < RCH && eb + threadIdx.x < e1) {
                 double t = 0.0;
-                for (int q = 0; q < RSPL; ++q) t += s_part[q * RCH + threadIdx.x];
+                for (int q = 0; q < RSPL / 2; ++q) t += s_part[q * RCH + threadIdx.x];
                 red[eb + threadIdx.x] = t;
             }
             __syncthreads();
@@ -232,6 +234,7 @@ __device__ inline void g_mm(double* C, int ldc, const double* A, int lda, bool t
     for (int e = threadIdx.x; e < m * n; e += NT) {
         const int i = e / n, j = e - (e / n) * n;
         double s = 0.0;
+#pragma unroll 8
         for (int l = 0; l < k; ++l) {
             const double a = ta ? A[l * lda + i] : A[i * lda + l];
             const double bb = tb ? B[j * ldb + l] : B[l * ldb + j];

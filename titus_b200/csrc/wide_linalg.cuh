@@ -32,51 +32,79 @@ static __device__ __noinline__ double cta_sum(double v) {
 // Upper Cholesky of G (k x k, ld ldg, any memory) into R (shared, ld) and its
 // inverse Ri (shared, ld). Returns ||R||_F ||R^{-1}||_F, or +inf on a
 // non-positive pivot; *ri_f receives ||R^{-1}||_F (a bound 1/sigma_min).
+// Elimination without square roots: the row operations that make G = L D L^T
+// upper triangular are applied to the identity as well (its rows grow in the
+// part of R below the diagonal), so that L^{-1} is there when the last pivot is;
+// R = D^{1/2} L^T and R^{-1} = L^{-T} D^{-1/2} are scaled at the end, all entries
+// at once. What bounds it is the chain of one step (pivot load, reciprocal,
+// product, update, barrier). The step has no loop of unknown length: the
+// unrolled prologue of one costs 300 cycles, as much as the chain. The
+// column-by-column form (square root, division and three barriers a step, then k
+// dependent dot products a column for the inverse) took 2100 cycles a step at
+// k = 17.
 static __device__ __noinline__ double w_chol(const double* G, int ldg, double* R, double* Ri, int ld, int k,
                                              double* ri_f) {
-    __shared__ int s_ok;
+    __builtin_assume(__isShared(R));
+    __builtin_assume(__isShared(Ri));
     __shared__ double s_nr[NT / 32], s_ni[NT / 32];
-    for (int e = threadIdx.x; e < k * k; e += NT) {
-        const int i = e / k, j = e - (e / k) * k;
-        R[i * ld + j] = (j >= i) ? G[i * ldg + j] : 0.0;
-        Ri[i * ld + j] = 0.0;
-    }
-    if (threadIdx.x == 0) s_ok = 1;
-    __syncthreads();
-    for (int j = 0; j < k; ++j) {
-        const double d = R[j * ld + j];
-        const bool okp = d > 0.0;
-        const double piv = okp ? sqrt(d) : 1.0;
-        __syncthreads();
-        for (int l = j + threadIdx.x; l < k; l += NT) R[j * ld + l] = (l == j) ? piv : R[j * ld + l] / piv;
-        if (!okp && threadIdx.x == 0) s_ok = 0;
-        __syncthreads();
-        const int m = k - j - 1;
-        for (int e = threadIdx.x; e < m * m; e += NT) {
-            const int i = j + 1 + e / m, l = j + 1 + (e - (e / m) * m);
-            if (l >= i) R[i * ld + l] = fma(-R[j * ld + i], R[j * ld + l], R[i * ld + l]);
-        }
-        __syncthreads();
-    }
-    // R^{-1}: warp w solves columns c = w, w+8, ...; lanes split each dot product
+    constexpr int WARPS = NT / 32, ROWS = (RA + WARPS - 1) / WARPS, COLS = (RA + 31) / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = warp; c < k; c += NT / 32) {
-        if (lane == 0) Ri[c * ld + c] = 1.0 / R[c * ld + c];
-        __syncwarp();
-        for (int a = c - 1; a >= 0; --a) {
-            double s = 0.0;
-            for (int bb = a + 1 + lane; bb <= c; bb += 32) s = fma(R[a * ld + bb], Ri[bb * ld + c], s);
-            s = warp_sum(s);
-            if (lane == 0) Ri[a * ld + c] = -s / R[a * ld + a];
-            __syncwarp();
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u)
+#pragma unroll
+        for (int h = 0; h < COLS; ++h) {
+            const int i = warp + u * WARPS, l = lane + 32 * h;
+            if (i < k && l < k) R[i * ld + l] = l >= i ? G[i * ldg + l] : 0.0;
         }
+    __syncthreads();
+    bool ok = true;
+#pragma unroll 1
+    for (int j = 0; j < k - 1; ++j) {
+        const double d = R[j * ld + j];
+        ok = ok && d > 0.0;
+        const double inv = -1.0 / (d > 0.0 ? d : 1.0);
+        double rj[COLS];
+#pragma unroll
+        for (int h = 0; h < COLS; ++h) rj[h] = R[j * ld + min(lane + 32 * h, k - 1)];
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+            const int i = j + 1 + warp + u * WARPS;
+            if (i < k) {
+                const double f = R[j * ld + i] * inv;
+#pragma unroll
+                for (int h = 0; h < COLS; ++h) {
+                    const int l = lane + 32 * h;
+                    // columns l >= i: U; l < j: the identity's rows, whose entry j is f itself
+                    if (l < k && (l >= i || l <= j))
+                        R[i * ld + l] = l == j ? f : fma(f, rj[h], R[i * ld + l]);
+                }
+            }
+        }
+        __syncthreads();
     }
+    ok = ok && R[(k - 1) * ld + k - 1] > 0.0;
     __syncthreads();
     double nr = 0.0, ni = 0.0;
-    for (int e = threadIdx.x; e < k * k; e += NT) {
-        const int i = e / k, j = e - (e / k) * k;
-        nr = fma(R[i * ld + j], R[i * ld + j], nr);
-        ni = fma(Ri[i * ld + j], Ri[i * ld + j], ni);
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+        const int i = warp + u * WARPS;
+        if (i < k) {
+            const double di = R[i * ld + i];
+            const double piv = di > 0.0 ? sqrt(di) : 1.0;
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < COLS; ++h) {
+                const int l = lane + 32 * h;
+                if (l < k) {
+                    const double v = l == i ? piv : R[i * ld + l] / piv;
+                    const double w = l == i ? 1.0 / piv : v;
+                    R[i * ld + l] = l >= i ? v : 0.0;
+                    Ri[l * ld + i] = l <= i ? w : 0.0;
+                    nr = l >= i ? fma(v, v, nr) : nr;
+                    ni = l <= i ? fma(w, w, ni) : ni;
+                }
+            }
+        }
     }
     nr = warp_sum(nr);
     ni = warp_sum(ni);
@@ -86,11 +114,11 @@ static __device__ __noinline__ double w_chol(const double* G, int ldg, double* R
     }
     __syncthreads();
     double tr = 0.0, ti = 0.0;
+#pragma unroll
     for (int w = 0; w < NT / 32; ++w) {
         tr += s_nr[w];
         ti += s_ni[w];
     }
-    const bool ok = s_ok != 0;
     __syncthreads();
     if (ri_f) *ri_f = ok ? sqrt(ti) : INFINITY;
     return ok ? sqrt(tr) * sqrt(ti) : INFINITY;
@@ -106,8 +134,11 @@ static __device__ __noinline__ double w_chol(const double* G, int ldg, double* R
 // separated directions use a negligible floor.
 static __device__ __noinline__ int w_eig(double* A, double* V, int ld, double* lam, int k, int* status,
                                          double rel_floor, double rel_tol = 1e-15) {
-    __shared__ double rc[RA / 2 + 1], rs[RA / 2 + 1], rdp[RA / 2 + 1], rdq[RA / 2 + 1];
-    __shared__ int rp[RA / 2 + 1], rq[RA / 2 + 1];
+    __builtin_assume(__isShared(A));
+    __builtin_assume(__isShared(V));
+    // rotations of a round: (cos, sin), the rotated diagonal, the pair (q = -1: p stays put)
+    __shared__ double2 s_cs[RA / 2 + 1], s_dd[RA / 2 + 1];
+    __shared__ int2 s_pq[RA / 2 + 1];
     __shared__ int s_rot[2];
     __shared__ double s_lam[RA];
     __shared__ int s_perm[RA];
@@ -118,6 +149,8 @@ static __device__ __noinline__ int w_eig(double* A, double* V, int ld, double* l
         __syncthreads();
         return 0;
     }
+    // an odd k gets a zero row and column (ld >= k + 1): its pairs never rotate, and
+    // the other rotations leave it zero, so no update looks at the padding
     const int m = k + (k & 1);
     const int npairs = m / 2;
     __shared__ double s_floor;
@@ -126,46 +159,58 @@ static __device__ __noinline__ int w_eig(double* A, double* V, int ld, double* l
         for (int i = 0; i < k; ++i) mx = fmax(mx, fabs(A[i * ld + i]));
         s_floor = rel_floor * mx;
     }
+    if (m > k && threadIdx.x < m) {
+        A[threadIdx.x * ld + k] = A[k * ld + threadIdx.x] = 0.0;
+        V[threadIdx.x * ld + k] = 0.0;
+    }
     __syncthreads();
     const double afloor = s_floor;
+    // This thread's share of a round's updates, fixed over the rounds: the 2 x 2
+    // blocks (a, b) of A, then the row segments (pair b, row i) of V, dealt to all
+    // threads in one list so that a round is one pass between its barriers.
+    constexpr int MAXW = ((RA / 2) * (RA / 2) + (RA / 2) * RA + NT - 1) / NT;
+    int wk[MAXW];
+#pragma unroll
+    for (int u = 0; u < MAXW; ++u) {
+        const int e = threadIdx.x + u * NT, v = e - npairs * npairs;
+        wk[u] = -1;
+        if (v < 0) wk[u] = (e / npairs) << 8 | (e - (e / npairs) * npairs);
+        else if (v < npairs * k) wk[u] = 1 << 16 | (v / k) << 8 | (v - (v / k) * k);
+    }
     bool conv = false;
     int nsw = 60;
+#pragma unroll 1
     for (int sweep = 0; sweep < 60; ++sweep) {
         const int par = sweep & 1;
         if (threadIdx.x == 0) s_rot[par] = 0;
         __syncthreads();
+#pragma unroll 1
         for (int t = 0; t < m - 1; ++t) {
             if (threadIdx.x < npairs) {
                 int p, q;
+                rr_pair(m, t, threadIdx.x, k, p, q);
                 double c = 1.0, s = 0.0;
-                if (rr_pair(m, t, threadIdx.x, k, p, q)) {
-                    const double apq = A[p * ld + q];
-                    const double app = A[p * ld + p], aqq = A[q * ld + q];
-                    // a rotation whose angle is below eps changes nothing (|a_pq| <= eps max|a|):
-                    // skipping it keeps the sweep count finite on rounding-level entries
-                    if (fabs(apq) > afloor && apq * apq > rel_tol * rel_tol * fabs(app * aqq) &&
-                        fabs(apq) > 4.4e-16 * fmax(fabs(app), fabs(aqq))) {
-                        // t = tan of the rotation angle, the smaller root of
-                        // t^2 + 2 th t - 1 = 0 with th = (aqq - app) / (2 apq), in the
-                        // form t = 2 apq sgn(d) / (|d| + sqrt(d^2 + 4 apq^2)), d = aqq - app
-                        const double d = aqq - app;
-                        const double tt = 2.0 * apq * copysign(1.0, d) / (fabs(d) + sqrt(fma(d, d, 4.0 * apq * apq)));
-                        c = rsqrt(fma(tt, tt, 1.0));
-                        s = tt * c;
-                        // the rotated 2x2 block in closed form (a_pq -> 0 exactly):
-                        // two-sided updates leave a_pq at a few eps max|a_pp|, |a_qq|,
-                        // which the next sweep would rotate again without end
-                        rdp[threadIdx.x] = fma(-tt, apq, app);
-                        rdq[threadIdx.x] = fma(tt, apq, aqq);
-                        s_rot[par] = 1;
-                    }
-                } else {
-                    q = -1;   // p is real, its partner the padding index: p stays put this round
+                const double apq = A[p * ld + q];
+                const double app = A[p * ld + p], aqq = A[q * ld + q];
+                // a rotation whose angle is below eps changes nothing (|a_pq| <= eps max|a|):
+                // skipping it keeps the sweep count finite on rounding-level entries
+                if (fabs(apq) > afloor && apq * apq > rel_tol * rel_tol * fabs(app * aqq) &&
+                    fabs(apq) > 4.4e-16 * fmax(fabs(app), fabs(aqq))) {
+                    // t = tan of the rotation angle, the smaller root of
+                    // t^2 + 2 th t - 1 = 0 with th = (aqq - app) / (2 apq), in the
+                    // form t = 2 apq sgn(d) / (|d| + sqrt(d^2 + 4 apq^2)), d = aqq - app
+                    const double d = aqq - app;
+                    const double tt = 2.0 * apq * copysign(1.0, d) / (fabs(d) + sqrt(fma(d, d, 4.0 * apq * apq)));
+                    c = rsqrt(fma(tt, tt, 1.0));
+                    s = tt * c;
+                    // the rotated 2x2 block in closed form (a_pq -> 0 exactly):
+                    // two-sided updates leave a_pq at a few eps max|a_pp|, |a_qq|,
+                    // which the next sweep would rotate again without end
+                    s_dd[threadIdx.x] = make_double2(fma(-tt, apq, app), fma(tt, apq, aqq));
+                    s_rot[par] = 1;
                 }
-                rc[threadIdx.x] = c;
-                rs[threadIdx.x] = s;
-                rp[threadIdx.x] = p;
-                rq[threadIdx.x] = q;
+                s_cs[threadIdx.x] = make_double2(c, s);
+                s_pq[threadIdx.x] = make_int2(p, q);
             }
             __syncthreads();
             // Both rotations at once: the thread owning rows {p_a, q_a} x columns
@@ -173,41 +218,33 @@ static __device__ __noinline__ int w_eig(double* A, double* V, int ld, double* l
             // columns by pair b (the order of the two one-sided passes) and writes
             // them back; no other thread touches them, so one barrier suffices.
             // A rotated diagonal block takes the closed form.
-            for (int e = threadIdx.x; e < npairs * npairs; e += NT) {
-                const int a = e / npairs, b = e - (e / npairs) * npairs;
-                const double sa = rs[a], sb = rs[b];
-                if (sa == 0.0 && sb == 0.0) continue;
-                const int pa = rp[a], qa = rq[a], pb = rp[b], qb = rq[b];
-                if (a == b) {
-                    A[pa * ld + pa] = rdp[a];
-                    A[qa * ld + qa] = rdq[a];
-                    A[pa * ld + qa] = 0.0;
-                    A[qa * ld + pa] = 0.0;
-                    continue;
+#pragma unroll
+            for (int u = 0; u < MAXW; ++u) {
+                if (wk[u] < 0) break;
+                const int hi = wk[u] >> 8 & 255, lo = wk[u] & 255;
+                const double2 csa = s_cs[hi];
+                const int2 pqa = s_pq[hi];
+                const double ca = csa.x, sa = csa.y;
+                const int pa = pqa.x, qa = pqa.y;
+                if (wk[u] >> 16) {
+                    const double vp = V[lo * ld + pa], vq = V[lo * ld + qa];
+                    V[lo * ld + pa] = ca * vp - sa * vq;
+                    V[lo * ld + qa] = sa * vp + ca * vq;
+                } else {
+                    const double2 csb = s_cs[lo], dd = s_dd[hi];
+                    const int2 pqb = s_pq[lo];
+                    const double cb = csb.x, sb = csb.y;
+                    const int pb = pqb.x, qb = pqb.y;
+                    const double xpp = A[pa * ld + pb], xpq = A[pa * ld + qb];
+                    const double xqp = A[qa * ld + pb], xqq = A[qa * ld + qb];
+                    const double rpp = ca * xpp - sa * xqp, rpq = ca * xpq - sa * xqq;
+                    const double rqp = sa * xpp + ca * xqp, rqq = sa * xpq + ca * xqq;
+                    const bool closed = hi == lo && sa != 0.0;
+                    A[pa * ld + pb] = closed ? dd.x : cb * rpp - sb * rpq;
+                    A[pa * ld + qb] = closed ? 0.0 : sb * rpp + cb * rpq;
+                    A[qa * ld + pb] = closed ? 0.0 : cb * rqp - sb * rqq;
+                    A[qa * ld + qb] = closed ? dd.y : sb * rqp + cb * rqq;
                 }
-                const double ca = rc[a], cb = rc[b];
-                const double xpp = A[pa * ld + pb];
-                const double xpq = qb >= 0 ? A[pa * ld + qb] : 0.0;
-                const double xqp = qa >= 0 ? A[qa * ld + pb] : 0.0;
-                const double xqq = (qa >= 0 && qb >= 0) ? A[qa * ld + qb] : 0.0;
-                const double rpp = ca * xpp - sa * xqp, rpq = ca * xpq - sa * xqq;
-                const double rqp = sa * xpp + ca * xqp, rqq = sa * xpq + ca * xqq;
-                A[pa * ld + pb] = cb * rpp - sb * rpq;
-                if (qb >= 0) A[pa * ld + qb] = sb * rpp + cb * rpq;
-                if (qa >= 0) {
-                    A[qa * ld + pb] = cb * rqp - sb * rqq;
-                    if (qb >= 0) A[qa * ld + qb] = sb * rqp + cb * rqq;
-                }
-            }
-            for (int e = threadIdx.x; e < npairs * k; e += NT) {
-                const int b = e / k, i = e - (e / k) * k;
-                const double sb = rs[b];
-                if (sb == 0.0) continue;
-                const int pb = rp[b], qb = rq[b];
-                const double cb = rc[b];
-                const double vp = V[i * ld + pb], vq = V[i * ld + qb];
-                V[i * ld + pb] = cb * vp - sb * vq;
-                V[i * ld + qb] = sb * vp + cb * vq;
             }
             __syncthreads();
         }
@@ -242,18 +279,96 @@ static __device__ __noinline__ int w_eig(double* A, double* V, int ld, double* l
     return nsw;
 }
 
+// The sweeps of w_svd with LP lanes per column pair (m <= 3 LP). Returns the
+// number of sweeps, or -1 without convergence.
+template <int LP>
+__device__ __forceinline__ int svd_sweeps(double* At, double* Vt, int ld, int m, double ctol, double nfloor,
+                                          int* s_rot) {
+    constexpr int PPW = 32 / LP;   // pairs per warp
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int mm = m + (m & 1);
+    const int npairs = mm / 2;
+    const int grp = lane / LP, gl = lane % LP;
+#pragma unroll 1
+    for (int sweep = 0; sweep < 60; ++sweep) {
+        const int par = sweep & 1;
+        if (threadIdx.x == 0) s_rot[par] = 0;
+        __syncthreads();
+#pragma unroll 1
+        for (int t = 0; t < mm - 1; ++t) {
+            // warp-uniform loop; every lane runs the shuffles
+#pragma unroll 1
+            for (int sb = warp * PPW; sb < npairs; sb += (NT / 32) * PPW) {
+                const int sidx = sb + grp;
+                int p = 0, q = 0;
+                const bool valid = sidx < npairs && rr_pair(mm, t, sidx, m, p, q);
+                // both columns, and those of V, stay in registers from the dot products to
+                // the update: one shared-memory latency a round instead of one per element
+                double uu[3], vv[3], wu[3], wv[3];
+                double a = 0.0, bq = 0.0, g = 0.0;
+#pragma unroll
+                for (int h = 0; h < 3; ++h) {
+                    const int i = gl + h * LP;
+                    const bool in = valid && i < m;
+                    uu[h] = in ? At[p * ld + i] : 0.0;
+                    vv[h] = in ? At[q * ld + i] : 0.0;
+                    wu[h] = in ? Vt[p * ld + i] : 0.0;
+                    wv[h] = in ? Vt[q * ld + i] : 0.0;
+                }
+#pragma unroll
+                for (int h = 0; h < 3; ++h) {
+                    a = fma(uu[h], uu[h], a);
+                    bq = fma(vv[h], vv[h], bq);
+                    g = fma(uu[h], vv[h], g);
+                }
+#pragma unroll
+                for (int o = LP / 2; o > 0; o >>= 1) {
+                    a += __shfl_xor_sync(0xffffffffu, a, o);
+                    bq += __shfl_xor_sync(0xffffffffu, bq, o);
+                    g += __shfl_xor_sync(0xffffffffu, g, o);
+                }
+                // skip rotations with an angle below eps (no effect on the columns)
+                if (valid && g != 0.0 && fmin(a, bq) > nfloor && g * g > ctol * ctol * a * bq &&
+                    fabs(g) > 2.2e-16 * fmax(a, bq)) {
+                    // t = tan of the angle orthogonalising the two columns:
+                    // t = 2 g sgn(d) / (|d| + sqrt(d^2 + 4 g^2)), d = |y|^2 - |x|^2
+                    const double d = bq - a;
+                    const double tt = 2.0 * g * copysign(1.0, d) / (fabs(d) + sqrt(fma(d, d, 4.0 * g * g)));
+                    const double c = rsqrt(fma(tt, tt, 1.0)), sn = c * tt;
+#pragma unroll
+                    for (int h = 0; h < 3; ++h) {
+                        const int i = gl + h * LP;
+                        if (i < m) {
+                            At[p * ld + i] = c * uu[h] - sn * vv[h];
+                            At[q * ld + i] = sn * uu[h] + c * vv[h];
+                            Vt[p * ld + i] = c * wu[h] - sn * wv[h];
+                            Vt[q * ld + i] = sn * wu[h] + c * wv[h];
+                        }
+                    }
+                    if (gl == 0) s_rot[par] = 1;
+                }
+            }
+            __syncthreads();
+        }
+        if (!s_rot[par]) return sweep + 1;
+    }
+    return -1;
+}
+
 // One-sided Jacobi SVD of the m x m matrix whose column p is At[p*ld .. +m)
 // (transposed storage keeps column operations on contiguous shared memory).
 // On return At[p] = sigma_p u_p and Vt[p] = v_p (unsorted); sig[j] and
 // perm[j] list the singular values in descending order (sigma_j = sig[j],
 // column perm[j]). Returns the number of sweeps, or -1 without convergence.
 static __device__ __noinline__ int w_svd(double* At, double* Vt, int ld, int m, double* sig, int* perm) {
+    __builtin_assume(__isShared(At));
+    __builtin_assume(__isShared(Vt));
     __shared__ int s_rot[2];
     __shared__ double s_n[KA];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int e = threadIdx.x; e < m * m; e += NT) Vt[(e / m) * ld + e % m] = ((e / m) == (e % m)) ? 1.0 : 0.0;
     __syncthreads();
-    int sweeps = -1;
+    int sweeps = 0;
     // rotation threshold: a recomputed dot product of two length-m columns
     // carries rounding of about m eps |x| |y|. Columns with |x| below
     // 1e-16 ||A||_F are numerically null and not rotated. (A floor as high as
@@ -269,65 +384,10 @@ static __device__ __noinline__ int w_svd(double* At, double* Vt, int ld, int m, 
     }
     __syncthreads();
     const double nfloor = 1e-32 * s_fro;
-    if (m > 1) {
-        const int mm = m + (m & 1);
-        const int npairs = mm / 2;
-        // LP lanes per pair (8 / 16 / 32), PPW = 32 / LP pairs per warp
-        const int LP = m <= 24 ? 8 : (m <= 48 ? 16 : 32);
-        const int PPW = 32 / LP;
-        const int grp = lane / LP, gl = lane % LP;
-        for (int sweep = 0; sweep < 60; ++sweep) {
-            const int par = sweep & 1;
-            if (threadIdx.x == 0) s_rot[par] = 0;
-            __syncthreads();
-            for (int t = 0; t < mm - 1; ++t) {
-                // warp-uniform loop; every lane runs the shuffles
-                for (int sb = warp * PPW; sb < npairs; sb += (NT / 32) * PPW) {
-                    const int sidx = sb + grp;
-                    int p = 0, q = 0;
-                    const bool valid = sidx < npairs && rr_pair(mm, t, sidx, m, p, q);
-                    double a = 0.0, bq = 0.0, g = 0.0;
-                    if (valid)
-                        for (int i = gl; i < m; i += LP) {
-                            const double u = At[p * ld + i], v = At[q * ld + i];
-                            a = fma(u, u, a);
-                            bq = fma(v, v, bq);
-                            g = fma(u, v, g);
-                        }
-                    for (int o = LP / 2; o > 0; o >>= 1) {
-                        a += __shfl_xor_sync(0xffffffffu, a, o);
-                        bq += __shfl_xor_sync(0xffffffffu, bq, o);
-                        g += __shfl_xor_sync(0xffffffffu, g, o);
-                    }
-                    // skip rotations with an angle below eps (no effect on the columns)
-                    if (valid && g != 0.0 && fmin(a, bq) > nfloor && g * g > ctol * ctol * a * bq &&
-                        fabs(g) > 2.2e-16 * fmax(a, bq)) {
-                        // t = tan of the angle orthogonalising the two columns:
-                        // t = 2 g sgn(d) / (|d| + sqrt(d^2 + 4 g^2)), d = |y|^2 - |x|^2
-                        const double d = bq - a;
-                        const double tt = 2.0 * g * copysign(1.0, d) / (fabs(d) + sqrt(fma(d, d, 4.0 * g * g)));
-                        const double c = rsqrt(fma(tt, tt, 1.0)), sn = c * tt;
-                        for (int i = gl; i < m; i += LP) {
-                            const double u = At[p * ld + i], v = At[q * ld + i];
-                            At[p * ld + i] = c * u - sn * v;
-                            At[q * ld + i] = sn * u + c * v;
-                            const double vu = Vt[p * ld + i], vv = Vt[q * ld + i];
-                            Vt[p * ld + i] = c * vu - sn * vv;
-                            Vt[q * ld + i] = sn * vu + c * vv;
-                        }
-                        if (gl == 0) s_rot[par] = 1;
-                    }
-                }
-                __syncthreads();
-            }
-            if (!s_rot[par]) {
-                sweeps = sweep + 1;
-                break;
-            }
-        }
-    } else {
-        sweeps = 0;
-    }
+    static_assert(KA <= 96, "three elements of a column per lane");
+    if (m > 48) sweeps = svd_sweeps<32>(At, Vt, ld, m, ctol, nfloor, s_rot);
+    else if (m > 24) sweeps = svd_sweeps<16>(At, Vt, ld, m, ctol, nfloor, s_rot);
+    else if (m > 1) sweeps = svd_sweeps<8>(At, Vt, ld, m, ctol, nfloor, s_rot);
     // singular values and descending order (stable)
     for (int p = warp; p < m; p += NT / 32) {
         double a = 0.0;
