@@ -40,38 +40,41 @@ __device__ inline void w_stencil(const WCtx& x, const double* A, int lda, int r0
     const DevProblem& P = x.P;
     const double hx = 0.5 / P.dx, hy = 0.5 / P.dy;
     const double ix = 1.0 / P.dx, iy = 1.0 / P.dy;
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        const int r = e / k, j = e - (e / k) * k;
-        const int c = r0 + r;
-        double l2x = 0.0, l2y = 0.0, l1x = 0.0, l1y = 0.0, l2z = 0.0, l1z = 0.0;
-        if (!is_bnd_w(P, c)) {
-            const double* p = A + (size_t)c * lda + j;
-            const double a0 = ldcg(p) * __ldg(P.rinv + c);
-            const double axm = ldcg(p - (size_t)P.ny * lda) * __ldg(P.rinv + c - P.ny);
-            const double axp = ldcg(p + (size_t)P.ny * lda) * __ldg(P.rinv + c + P.ny);
-            const double aym = ldcg(p - lda) * __ldg(P.rinv + c - 1);
-            const double ayp = ldcg(p + lda) * __ldg(P.rinv + c + 1);
-            l2x = (axp - axm) * hx;
-            l2y = (ayp - aym) * hy;
-            l1x = a0 * ix - hx * axm - hx * axp;
-            l1y = a0 * iy - hy * aym - hy * ayp;
-            if constexpr (kThreeD) {
-                const int nxy = P.nx * P.ny;
-                const double hz = 0.5 / P.dz, iz = 1.0 / P.dz;
-                const double azm = ldcg(p - (size_t)nxy * lda) * __ldg(P.rinv + c - nxy);
-                const double azp = ldcg(p + (size_t)nxy * lda) * __ldg(P.rinv + c + nxy);
-                l2z = (azp - azm) * hz;
-                l1z = a0 * iz - hz * azm - hz * azp;
-            }
+    const int nxy = P.nx * P.ny;
+    const double hz = kThreeD ? 0.5 / P.dz : 0.0, iz = kThreeD ? 1.0 / P.dz : 0.0;
+    // two elements a thread at a time: the neighbours of both are in flight before either is used
+    constexpr int SU = 2, NB = kThreeD ? 7 : 5;
+    RowWalk it(k);
+#pragma unroll 1
+    while (it.r < nr) {
+        double a[SU][NB];
+        int rr[SU], jj[SU];
+        bool in[SU];
+#pragma unroll
+        for (int u = 0; u < SU; ++u) {
+            rr[u] = it.r;
+            jj[u] = it.j;
+            const int c = r0 + min(it.r, nr - 1);
+            in[u] = it.r < nr && !is_bnd_w(P, c);
+            const int off[7] = {0, -P.ny, P.ny, -1, 1, -nxy, nxy};
+            const double* p = A + (size_t)c * lda + it.j;
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+                a[u][b] = in[u] ? ldcg(p + (ptrdiff_t)off[b] * lda) * __ldg(P.rinv + c + off[b]) : 0.0;
+            it.next();
         }
-        double* row = F + r * ldf + fc;
-        row[0 * k + j] = l2x;
-        row[1 * k + j] = l2y;
-        row[2 * k + j] = l1x;
-        row[3 * k + j] = l1y;
-        if constexpr (kThreeD) {
-            row[4 * k + j] = l2z;
-            row[5 * k + j] = l1z;
+#pragma unroll
+        for (int u = 0; u < SU; ++u) {
+            if (rr[u] >= nr) break;
+            double* row = F + rr[u] * ldf + fc + jj[u];
+            row[0 * k] = (a[u][2] - a[u][1]) * hx;
+            row[1 * k] = (a[u][4] - a[u][3]) * hy;
+            row[2 * k] = a[u][0] * ix - hx * a[u][1] - hx * a[u][2];
+            row[3 * k] = a[u][0] * iy - hy * a[u][3] - hy * a[u][4];
+            if constexpr (kThreeD) {
+                row[4 * k] = (a[u][NB - 1] - a[u][NB - 2]) * hz;
+                row[5 * k] = a[u][0] * iz - hz * a[u][NB - 2] - hz * a[u][NB - 1];
+            }
         }
     }
 }
@@ -480,9 +483,9 @@ static __device__ __noinline__ bool w_phase_C(WCtx& x) {
         // K = X S - dE (L_d X) (S C_d) stacked; the two chains of each entry are
         // formed by the same thread (same micro-tile map in both calls)
         const double* Sm = sm->S;
-        row_mm<4>(nr, k, k, T, ldT, [&](int l, int j) { return Sm[l * KA + j]; },
+        row_mm(nr, k, k, T, ldT, [&](int l, int j) { return Sm[l * KA + j]; },
                   [&](int r, int j, double v) { T[r * ldT + k + j] = v; });
-        row_mm<4>(nr, NOPS_W * k, k, F, ldF, [&](int l, int j) { return ST[l * k + j]; },
+        row_mm(nr, NOPS_W * k, k, F, ldF, [&](int l, int j) { return ST[l * k + j]; },
                   [&](int r, int j, double v) { T[r * ldT + k + j] = T[r * ldT + k + j] - dE * v; });
         __syncthreads();
         wstore(x.st.K, RA, 0, T, ldT, k, r0, nr, k);
@@ -499,9 +502,9 @@ static __device__ __noinline__ bool w_phase_C(WCtx& x) {
         __syncthreads();
         // L = W S^T - dE (A_d W) (S^T G_d^T) stacked
         const double* Sm = sm->S;
-        row_mm<4>(nr, k, k, T, ldT, [&](int l, int j) { return Sm[j * KA + l]; },
+        row_mm(nr, k, k, T, ldT, [&](int l, int j) { return Sm[j * KA + l]; },
                   [&](int r, int j, double v) { T[r * ldT + k + j] = v; });
-        row_mm<4>(nr, NOPS_W * k, k, F, ldF, [&](int l, int j) { return ST[l * k + j]; },
+        row_mm(nr, NOPS_W * k, k, F, ldF, [&](int l, int j) { return ST[l * k + j]; },
                   [&](int r, int j, double v) { T[r * ldT + k + j] = T[r * ldT + k + j] - dE * v; });
         __syncthreads();
         wstore(x.st.L, RA, 0, T, ldT, k, r0, nr, k);
@@ -648,7 +651,7 @@ static __device__ __noinline__ void aug_pass(WCtx& x, int s, bool second, double
         wload(F, ldF, 0, sb.A, KA, 0, r0, nr, k);
         wload(F, ldF, k, Bsrc, RA, 0, r0, nr, k);
         __syncthreads();
-        row_mm<4>(nr, k, k, F, ldF, [&](int l, int j) { return T[l * RA + j]; },
+        row_mm(nr, k, k, F, ldF, [&](int l, int j) { return T[l * RA + j]; },
                   [&](int r, int j, double v) { F[r * ldF + k + j] -= v; });
         __syncthreads();
         wstore(sb.BP, RA, 0, F, ldF, k, r0, nr, k);
@@ -680,19 +683,7 @@ static __device__ __noinline__ bool aug_project(WCtx& x) {
     return wreduce(x, 2 * k * k);
 }
 
-// Row-wise triangular solve t[r,:] <- t[r,:] R^{-1} (R upper, shared, ld RA).
-__device__ __forceinline__ void w_rsolve(double* t, int ldt, const double* R, int nr, int k) {
-    for (int r = threadIdx.x; r < nr; r += NT) {
-        double* row = t + r * ldt;
-        for (int j = 0; j < k; ++j) {
-            double v = row[j];
-            for (int i = 0; i < j; ++i) v = fma(-row[i], R[i * RA + j], v);
-            row[j] = v / R[j * RA + j];
-        }
-    }
-}
-
-// C = BP M (mode 0: M = R0 by row solves; mode 1: M = T (k x rho), product) for
+// C = BP M (mode 0: M = R0^{-1}, upper triangular; mode 1: M = T (k x rho)) for
 // own rows; acc[off..] += C^T C (rho x rho), or (mode 2) (BP V0)^T (BP V0) and
 // (mode 3) (A V0)^T (A V0) without storing C.
 static __device__ __noinline__ void rf_pass(WCtx& x, int s, int mode, int rho, double* acc, int off) {
@@ -711,14 +702,8 @@ static __device__ __noinline__ void rf_pass(WCtx& x, int s, int mode, int rho, d
         if (mode == 3) wload(F, ldF, 0, sb.A, KA, 0, r0, nr, k);
         else wload(F, ldF, 0, sb.BP, RA, 0, r0, nr, k);
         __syncthreads();
-        if (mode == 0) {
-            for (int e = threadIdx.x; e < nr * k; e += NT) F[(e / k) * ldF + k + e % k] = F[(e / k) * ldF + e % k];
-            __syncthreads();
-            w_rsolve(F + k, ldF, M, nr, k);
-        } else {
-            row_mm<4>(nr, k, w, F, ldF, [&](int l, int j) { return M[l * RA + j]; },
-                      [&](int r, int j, double v) { F[r * ldF + k + j] = v; });
-        }
+        row_mm(nr, k, w, F, ldF, [&](int l, int j) { return M[l * RA + j]; },
+               [&](int r, int j, double v) { F[r * ldF + k + j] = v; });
         __syncthreads();
         if (mode < 2) wstore(sb.C, RA, 0, F, ldF, k, r0, nr, w);
         gram_blocks(acc, F, ldF, nr, &bl, 1);
@@ -784,7 +769,7 @@ static __device__ __noinline__ void rf_slow_rank(WCtx& x, int s, int off, bool p
 // at offsets s*k^2. `plain[s]`: the rank cut is relative to the largest
 // singular value of BP itself (orth), else to side[s].scale (augmentation).
 //  certified path: Cholesky of BP^T BP with ||R||_F ||R^-1||_F < 1e5 (and, for
-//    augmentation, sigma_min > 10 tol scale): C = BP R0^{-1} by row solves;
+//    augmentation, sigma_min > 10 tol scale): C = BP R0^{-1};
 //  rank-revealing path: Jacobi of BP^T BP -> V0; Gram of BP V0 -> Jacobi ->
 //    V2, nu; C = BP V0 V2_J / nu_J for nu_j above the cut.
 // On return side[s].rho2 is set and SS_RI holds R^{-1} of the CholQR of C, so
@@ -811,7 +796,7 @@ static __device__ __noinline__ bool range_find(WCtx& x, const bool do_side[2], c
         if (ok) {
             si.fast2 = 1;
             si.rho2 = k;
-            g_copy(sside(x, s, SS_R0), RA, R, RA, k, k);
+            g_copy(sside(x, s, SS_R0), RA, Ri, RA, k, k);
         } else {
             si.fast2 = 0;
             slow[s] = true;
@@ -959,10 +944,10 @@ static __device__ __noinline__ void materialize_side(WCtx& x, int s, bool with_q
         if (rho2 > 0) wload(cb, LC, 0, sb.C, RA, 0, r0, nr, rho2);
         __syncthreads();
         // Q1 columns: range part A F1, then completion (X side only: the W side has rho1 == k)
-        row_mm<4>(nr, k, rho1, t, LT, [&](int l, int j) { return F1[l * RA + j]; },
+        row_mm(nr, k, rho1, t, LT, [&](int l, int j) { return F1[l * RA + j]; },
                   [&](int r, int j, double v) { t[r * LT + k + j] = v; });
         // X~ range part C RI (RI upper triangular: the terms l > j add exact zeros)
-        row_mm<4>(nr, rho2, rho2, cb, LC, [&](int l, int j) { return l <= j ? Ri[l * RA + j] : 0.0; },
+        row_mm(nr, rho2, rho2, cb, LC, [&](int l, int j) { return l <= j ? Ri[l * RA + j] : 0.0; },
                   [&](int r, int j, double v) { t[r * LT + 2 * k + j] = v; });
         for (int e = threadIdx.x; e < nr * k; e += NT) {
             const int r = e / k, j = e - (e / k) * k;
@@ -1139,7 +1124,7 @@ static __device__ __noinline__ void w_truncate_apply(WCtx& x, int m, int kk, int
             wload(t, ldt, 0, A, KA, 0, r0, nr, m);
             __syncthreads();
             const int* perm = sm->perm;
-            row_mm<4>(nr, m, kk, t, ldt, [&](int l, int j) { return B[perm[j] * LDS + l]; },
+            row_mm(nr, m, kk, t, ldt, [&](int l, int j) { return B[perm[j] * LDS + l]; },
                       [&](int r, int j, double v) { o[r * ldt + j] = v; });
             __syncthreads();
             wstore(A, KA, 0, o, ldt, 0, r0, nr, kk);
@@ -1178,7 +1163,7 @@ static __device__ __noinline__ bool w_outscatter_pass(WCtx& x, const double* sig
         wload(t, ldt, 0, x.st.W, KA, 0, r0, nr, k);
         __syncthreads();
         const double* Sm = sm->S;
-        row_mm<4>(nr, k, k, t, ldt, [&](int l, int j) { return Sm[j * KA + l]; }, [&](int r, int j, double v) {
+        row_mm(nr, k, k, t, ldt, [&](int l, int j) { return Sm[j * KA + l]; }, [&](int r, int j, double v) {
             const double D = sig[0] - sig[P.lof[r0 + r]];
             t[r * ldt + k + j] = v / (1.0 + P.dE * D);
         });
@@ -1230,7 +1215,7 @@ static __device__ __noinline__ bool w_outscatter_basis(WCtx& x, const double* si
             t[r * ldt + 3 * RA + kq] = P.mred[(size_t)m * P.q + kq] * sig[P.lof[m]];
         }
         __syncthreads();
-        row_mm<4>(nr, rho, rho, t, ldt, [&](int l, int j) { return l <= j ? Ri[l * RA + j] : 0.0; },
+        row_mm(nr, rho, rho, t, ldt, [&](int l, int j) { return l <= j ? Ri[l * RA + j] : 0.0; },
                   [&](int r, int j, double v) { t[r * ldt + RA + j] = v; });
         __syncthreads();
         if (k > rho) {
@@ -1325,9 +1310,9 @@ static __device__ __noinline__ bool w_inscatter_KL(WCtx& x, const double* sig, b
         __syncthreads();
         // K = X S + dE psi MtDW (zero on boundary rows), two chains per entry
         const double* Sm = sm->S;
-        row_mm<4>(nr, k, k, t, ldt, [&](int l, int j) { return Sm[l * KA + j]; },
+        row_mm(nr, k, k, t, ldt, [&](int l, int j) { return Sm[l * KA + j]; },
                   [&](int r, int j, double v) { t[r * ldt + k + j] = is_bnd_w(P, r0 + r) ? 0.0 : v; });
-        row_mm<4>(nr, P.q, k, t + 2 * k, ldt, [&](int l, int j) { return Mt[l * KA + j]; },
+        row_mm(nr, P.q, k, t + 2 * k, ldt, [&](int l, int j) { return Mt[l * KA + j]; },
                   [&](int r, int j, double v) {
                       if (!is_bnd_w(P, r0 + r)) t[r * ldt + k + j] += dE * v;
                   });

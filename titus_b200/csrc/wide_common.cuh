@@ -33,7 +33,11 @@ constexpr int NOPS_W = TITUS_WIDE_NOPS;
 constexpr bool kThreeD = NOPS_W == 6;
 static_assert(NOPS_W == 4 || NOPS_W == 6, "four (2D) or six (3D) streaming pairs");
 
-constexpr int NT = 512;   // threads per CTA
+// Threads per CTA. 512 against 256 (the same code, 148 CTAs unless stated): 200 x 200,
+// P29, ranks 8 to 20: 2616 and 2607 us a step; 128 x 128, P21: 2118 and 2316, on
+// one CTA (the batched form) 31.6 and 38.3 ms; 48 x 48, P7, ranks 2 to 9: 540 and
+// 521. The row work and the wide factorisations gain, the barriers lose a little.
+constexpr int NT = 512;
 constexpr int RA = titus::WIDE_RA;   // max rank entering a step
 constexpr int KA = 2 * RA;      // max augmented width
 constexpr int LDS = KA + 1;     // row stride of the truncation SVD's column arrays (odd: no bank conflicts)
@@ -68,7 +72,7 @@ enum : int {
     SS_P1 = SS_F1 + RA * RA,   // F1 F1^T
     SS_T = SS_P1 + RA * RA,    // projection coefficients / range-finder transform
     SS_M1 = SS_T + RA * RA,    // Q1^T A (BUG: top block of X1^T X)
-    SS_R0 = SS_M1 + RA * RA,   // Cholesky factor of the range-finder Gram
+    SS_R0 = SS_M1 + RA * RA,   // inverse Cholesky factor of the range-finder Gram
     SS_RI = SS_R0 + RA * RA,   // inverse Cholesky factor of C^T C (basis = C RI)
     SS_V0 = SS_RI + RA * RA,   // slow path: eigenvectors of G0
     SS_WC = SS_V0 + RA * RA,   // W-side completion coefficients (RA rows, stride WCS)
@@ -278,78 +282,104 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// This thread's elements of a nr x w tile in row order, NT apart: one division
+// at the start instead of one per element.
+struct RowWalk {
+    int r, j, w, dr, dj;
+    __device__ __forceinline__ explicit RowWalk(int w_) : w(w_) {
+        r = threadIdx.x / w;
+        j = threadIdx.x - r * w;
+        dr = NT / w;
+        dj = NT - dr * w;
+    }
+    __device__ __forceinline__ void next() {
+        r += dr;
+        j += dj;
+        if (j >= w) {
+            j -= w;
+            ++r;
+        }
+    }
+};
+
 // rows [r0, r0+nr) x cols [c0, c0+k) of A (ld lda) -> t (ld ldt) at column tc.
 // On return this thread's copies have landed; the caller's __syncthreads makes
 // the whole tile visible to the CTA.
 __device__ __forceinline__ void wload(double* t, int ldt, int tc, const double* A, int lda, int c0, int r0, int nr,
                                       int k) {
+    if (k <= 0) return;
     if (pairs_ok(t, A, k, c0, lda, ldt, tc)) {
-        const int h = k >> 1;
-        for (int e = threadIdx.x; e < nr * h; e += NT) {
-            const int r = e / h, j = 2 * (e - r * h);
-            cp_async16(t + r * ldt + tc + j, A + (size_t)(r0 + r) * lda + c0 + j);
-        }
+#pragma unroll 1
+        for (RowWalk x(k >> 1); x.r < nr; x.next())
+            cp_async16(t + x.r * ldt + tc + 2 * x.j, A + (size_t)(r0 + x.r) * lda + c0 + 2 * x.j);
     } else {
-        for (int e = threadIdx.x; e < nr * k; e += NT) {
-            const int r = e / k, j = e - r * k;
-            cp_async8(t + r * ldt + tc + j, A + (size_t)(r0 + r) * lda + c0 + j);
-        }
+#pragma unroll 1
+        for (RowWalk x(k); x.r < nr; x.next())
+            cp_async8(t + x.r * ldt + tc + x.j, A + (size_t)(r0 + x.r) * lda + c0 + x.j);
     }
     cp_async_wait_all();
 }
 __device__ __forceinline__ void wstore(double* A, int lda, int c0, const double* t, int ldt, int tc, int r0, int nr,
                                        int k) {
+    if (k <= 0) return;
     if (pairs_ok(t, A, k, c0, lda, ldt, tc)) {
-        const int h = k >> 1;
-        for (int e = threadIdx.x; e < nr * h; e += NT) {
-            const int r = e / h, j = 2 * (e - r * h);
-            *reinterpret_cast<double2*>(A + (size_t)(r0 + r) * lda + c0 + j) =
-                *reinterpret_cast<const double2*>(t + r * ldt + tc + j);
-        }
+#pragma unroll 1
+        for (RowWalk x(k >> 1); x.r < nr; x.next())
+            *reinterpret_cast<double2*>(A + (size_t)(r0 + x.r) * lda + c0 + 2 * x.j) =
+                *reinterpret_cast<const double2*>(t + x.r * ldt + tc + 2 * x.j);
         return;
     }
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        const int r = e / k, j = e - r * k;
-        A[(size_t)(r0 + r) * lda + c0 + j] = t[r * ldt + tc + j];
-    }
+#pragma unroll 1
+    for (RowWalk x(k); x.r < nr; x.next()) A[(size_t)(r0 + x.r) * lda + c0 + x.j] = t[x.r * ldt + tc + x.j];
+}
+
+// D += A B on an 8 x 8 tile, four columns of A at a time (FP64 tensor pipe): a
+// lane holds A[lane / 4][lane % 4], B[lane % 4][lane / 4] and
+// D[lane / 4][2 (lane % 4) + {0, 1}].
+__device__ __forceinline__ void w_mma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
 }
 
 // Row products of a shared-memory tile: for rows r < nr and columns j < w,
-//   epi(r, j, sum_{l < kd} A[r * lda + l] * mget(l, j))
-// with one FMA chain per output in increasing l (the rounding of the plain
-// per-element loop). A thread owns a micro-tile of RB rows x 2 columns: per l it
-// reads RB entries of A and 2 of M for 2 RB independent FMAs, instead of two
-// shared loads per dependent FMA. Threads of a warp share rows (broadcast reads
-// of A) and take adjacent column pairs (consecutive entries of M).
-template <int RB, class MGet, class Epi>
+//   epi(r, j, sum_{l < kd} A[r * lda + l] * mget(l, j)).
+// A warp takes 16 rows x 8 columns and walks l in steps of four on the FP64
+// tensor pipe: per step two loads of A and one of M for 512 products, where a
+// thread's 4 x 2 micro-tile took six loads for eight. Entries with l >= kd are
+// replaced by zeros (the tile's other columns are not read); rows and columns
+// beyond the tile repeat its last ones and are dropped. The map from (r, j) to
+// threads depends on nr and w only, so a second call may update what the first
+// one's epi wrote.
+template <class MGet, class Epi>
 __device__ __forceinline__ void row_mm(int nr, int kd, int w, const double* A, int lda, MGet mget, Epi epi) {
-    const int cb = (w + 1) >> 1, rbn = (nr + RB - 1) / RB;
-    for (int tile = threadIdx.x; tile < rbn * cb; tile += NT) {
-        const int rb = tile / cb, c2 = tile - rb * cb;
-        const int r0 = rb * RB, j0 = 2 * c2;
-        const bool j1 = j0 + 1 < w;
-        double acc[RB][2];
-#pragma unroll
-        for (int i = 0; i < RB; ++i) acc[i][0] = acc[i][1] = 0.0;
-        const double* ap[RB];
-#pragma unroll
-        for (int i = 0; i < RB; ++i) ap[i] = A + min(r0 + i, nr - 1) * lda;
-        for (int l = 0; l < kd; ++l) {
-            const double m0 = mget(l, j0);
-            const double m1 = j1 ? mget(l, j0 + 1) : 0.0;
-#pragma unroll
-            for (int i = 0; i < RB; ++i) {
-                const double a = ap[i][l];
-                acc[i][0] = fma(a, m0, acc[i][0]);
-                acc[i][1] = fma(a, m1, acc[i][1]);
-            }
+    if (w <= 0) return;
+    const int lane = threadIdx.x & 31, kr = lane & 3, ci = lane >> 2;
+    const int jt = (w + 7) >> 3, total = jt * ((nr + 15) >> 4);
+#pragma unroll 1
+    for (int it = threadIdx.x >> 5; it < total; it += NT / 32) {
+        const int rp = it / jt, j0 = 8 * (it - rp * jt), r0 = 16 * rp;
+        const double* a0 = A + min(r0 + ci, nr - 1) * lda;
+        const double* a1 = A + min(r0 + 8 + ci, nr - 1) * lda;
+        const int jb = min(j0 + ci, w - 1);
+        double d[2][2] = {};
+#pragma unroll 2
+        for (int l0 = 0; l0 < kd; l0 += 4) {
+            const int l = l0 + kr;
+            const bool in = l < kd;
+            const double b = in ? mget(l, jb) : 0.0;
+            const double x0 = in ? a0[l] : 0.0, x1 = in ? a1[l] : 0.0;
+            w_mma(d[0], x0, b);
+            w_mma(d[1], x1, b);
         }
 #pragma unroll
-        for (int i = 0; i < RB; ++i)
-            if (r0 + i < nr) {
-                epi(r0 + i, j0, acc[i][0]);
-                if (j1) epi(r0 + i, j0 + 1, acc[i][1]);
+        for (int h = 0; h < 2; ++h) {
+            const int r = r0 + 8 * h + ci, j = j0 + 2 * kr;
+            if (r < nr) {
+                if (j < w) epi(r, j, d[h][0]);
+                if (j + 1 < w) epi(r, j + 1, d[h][1]);
             }
+        }
     }
 }
 
@@ -357,66 +387,84 @@ __device__ __forceinline__ void row_mm(int nr, int kd, int w, const double* A, i
 struct GBlock {
     int ca, wa, cb, wb, off;
 };
-// Accumulate a list of blocks over a tile of nr rows; 2x2 register tiles. The
-// tiles of all blocks are flattened; each warp holds 32/G tiles in G row
-// subgroups (subgroup s sums rows s, s+G, ...; lanes of a subgroup share rows,
-// so their loads broadcast), G in {1, 2, 4, 8} minimising rounds x rows per
-// lane. The G partial sums of a tile meet in a fixed xor butterfly: the result
-// depends only on (blocks, nr), not on timing.
+// Accumulate a list of blocks over a tile of nr rows on the FP64 tensor pipe. An
+// item is 8 columns i x 16 columns j of one block; the items of all blocks are
+// dealt to the warps in list order, and where they leave warps over, 2 or 4
+// warps share an item's rows and add their sums one after the other, so the
+// result depends only on (blocks, nr), not on timing. Two accumulator sets per
+// tile (alternate row quads) keep dependent products apart. Columns beyond a
+// block are read (the tile's next ones, still inside the shared work area) into
+// entries that are not stored. Against a 2 x 2 register tile per thread, four
+// loads for four products, a step loads three values for 512.
 __device__ inline void gram_blocks(double* acc, const double* F, int ldf, int nr, const GBlock* bl, int nb) {
-    int T = 0;
-    for (int q = 0; q < nb; ++q) T += ((bl[q].wa + 1) >> 1) * ((bl[q].wb + 1) >> 1);
-    int G = 1, best = 0x7fffffff;
-    for (int g = 1; g <= 8; g <<= 1) {
-        const int slots = (NT / 32) * (32 / g);
-        const int cost = ((T + slots - 1) / slots) * ((nr + g - 1) / g);
-        if (cost < best) {
-            best = cost;
-            G = g;
-        }
-    }
-    const int L = 32 / G, slots = (NT / 32) * L;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int sg = lane / L, tl = lane - (lane / L) * L;
-    for (int base = 0; base < T; base += slots) {
-        int off = base + warp * L + tl;
-        const bool valid = off < T;
-        GBlock g{0, 2, 0, 2, 0};
-        int hj = 1;
-        if (valid)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kr = lane & 3, ci = lane >> 2;
+    constexpr int WARPS = NT / 32;
+    int total = 0;
+#pragma unroll 1
+    for (int q = 0; q < nb; ++q) total += ((bl[q].wa + 7) >> 3) * ((bl[q].wb + 15) >> 4);
+    const int parts = total * 4 <= WARPS ? 4 : total * 2 <= WARPS ? 2 : 1;
+#pragma unroll 1
+    for (int base = 0; base < total; base += WARPS / parts) {
+        int off = base + warp / parts;
+        const int part = warp & (parts - 1);
+        const bool valid = off < total;
+        GBlock g{0, 0, 0, 0, 0};
+        int tj = 1;
+        if (valid) {
+#pragma unroll 1
             for (int q = 0; q < nb; ++q) {
                 g = bl[q];
-                hj = (g.wb + 1) >> 1;
-                const int cnt = ((g.wa + 1) >> 1) * hj;
+                tj = (g.wb + 15) >> 4;
+                const int cnt = ((g.wa + 7) >> 3) * tj;
                 if (off < cnt) break;
                 off -= cnt;
             }
-        const int i = 2 * (off / hj), j = 2 * (off - (off / hj) * hj);
-        const bool i1 = i + 1 < g.wa, j1 = j + 1 < g.wb;
-        double s00 = 0.0, s01 = 0.0, s10 = 0.0, s11 = 0.0;
-        if (valid)
-            for (int r = sg; r < nr; r += G) {
-                const double* row = F + r * ldf;
-                const double a0 = row[g.ca + i], a1 = i1 ? row[g.ca + i + 1] : 0.0;
-                const double b0 = row[g.cb + j], b1 = j1 ? row[g.cb + j + 1] : 0.0;
-                s00 = fma(a0, b0, s00);
-                s01 = fma(a0, b1, s01);
-                s10 = fma(a1, b0, s10);
-                s11 = fma(a1, b1, s11);
-            }
-        for (int o = L; o < 32; o <<= 1) {
-            s00 += __shfl_xor_sync(0xffffffffu, s00, o);
-            s01 += __shfl_xor_sync(0xffffffffu, s01, o);
-            s10 += __shfl_xor_sync(0xffffffffu, s10, o);
-            s11 += __shfl_xor_sync(0xffffffffu, s11, o);
         }
-        if (valid && sg == 0) {
-            double* o = acc + g.off + i * g.wb + j;
-            o[0] += s00;
-            if (j1) o[1] += s01;
-            if (i1) {
-                o[g.wb] += s10;
-                if (j1) o[g.wb + 1] += s11;
+        const int i0 = 8 * (off / tj), j0 = 16 * (off - (off / tj) * tj);
+        const bool two = j0 + 8 < g.wb;
+        double d[2][2][2] = {};   // [row quad parity][column tile]
+        if (valid) {
+            const double* pa = F + kr * ldf + g.ca + i0 + ci;
+            const double* pb = F + kr * ldf + g.cb + j0 + ci;
+            const int step = 4 * parts * ldf;
+            int r = 4 * part;
+            pa += r * ldf;
+            pb += r * ldf;
+#pragma unroll 1
+            for (; r + 4 * parts + 4 <= nr; r += 8 * parts) {
+                const double x0 = pa[0], x1 = pa[step];
+                const double y0 = pb[0], y1 = pb[step];
+                w_mma(d[0][0], x0, y0);
+                w_mma(d[1][0], x1, y1);
+                if (two) {
+                    w_mma(d[0][1], x0, pb[8]);
+                    w_mma(d[1][1], x1, pb[step + 8]);
+                }
+                pa += 2 * step;
+                pb += 2 * step;
+            }
+#pragma unroll 1
+            for (; r < nr; r += 4 * parts) {
+                const bool in = r + kr < nr;
+                const double x0 = in ? pa[0] : 0.0, y0 = in ? pb[0] : 0.0, z0 = in && two ? pb[8] : 0.0;
+                w_mma(d[0][0], x0, y0);
+                if (two) w_mma(d[0][1], x0, z0);
+                pa += step;
+                pb += step;
+            }
+        }
+#pragma unroll 1
+        for (int p = 0; p < parts; ++p) {
+            if (p > 0) __syncthreads();
+            if (valid && part == p) {
+                const int i = i0 + ci;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int j = j0 + 8 * h + 2 * kr + u;
+                        if (i < g.wa && j < g.wb) acc[g.off + i * g.wb + j] += d[0][h][u] + d[1][h][u];
+                    }
             }
         }
     }
