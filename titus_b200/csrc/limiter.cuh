@@ -36,6 +36,23 @@ __device__ __forceinline__ double face_pos(double m1, double c, double p1) {
 __device__ __forceinline__ double face_neg(double m1, double c, double p1) {
     return __dsub_rn(c, __dmul_rn(0.5, slopefit(m1, c, p1)));
 }
+// The same faces from doubled differences that the caller forms once for two
+// neighbouring faces: dl = 2 (c - l), dr = 2 (r - c); face(l, c, r, dl, dr, true) =
+// face_pos(l, c, r), (..., false) = face_neg(l, c, r), the same IEEE doubles (the
+// products by 2 and the changes of sign are exact).
+__device__ __forceinline__ double twice_diff(double a, double b) { return __dmul_rn(2.0, __dsub_rn(b, a)); }
+// minmod with the sign of x moved to y: |y| outside [0, |x|] on either side
+__device__ __forceinline__ double minmod_s(double x, double y) {
+    const long long neg = x < 0.0 ? (long long)0x8000000000000000ull : 0ll;
+    const double ys = __longlong_as_double(__double_as_longlong(y) ^ neg);
+    const double r = ys > fabs(x) ? x : y;
+    return ys < 0.0 ? 0.0 : r;
+}
+__device__ __forceinline__ double face(double l, double c, double r, double dl, double dr, bool pos) {
+    const double s = minmod_s(dr, minmod_s(__dmul_rn(0.5, __dsub_rn(r, l)), dl));
+    const double h = __dmul_rn(0.5, s);
+    return __dadd_rn(c, pos ? h : -h);
+}
 // (face after the centre) - (face before it) along one axis from the five
 // values at offsets -2..+2 (only -2..+1 are read for pos, -1..+2 otherwise)
 __device__ __forceinline__ double axis_diff(double m2, double m1, double c, double p1, double p2, bool pos) {
