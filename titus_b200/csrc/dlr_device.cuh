@@ -12,10 +12,11 @@
 
 namespace titus {
 
-constexpr int NT = 256;        // threads per CTA
+constexpr int NT = 512;        // threads per CTA
+constexpr int NW = NT / 32;    // warps per CTA
 constexpr int KM = 24;         // max basis width handled by this build
 constexpr int QM = 32;         // max reduced ordinates
-constexpr int TR = 32;         // rows per staged tile
+constexpr int TR = 40;         // rows per staged tile: one pair of columns per thread
 constexpr int NOPS = 4;        // Ax, Az, |Ax|, |Az|
 constexpr int KK = KM * KM;
 constexpr int PMAX = 8 * KK;  // partial-reduction capacity (doubles); >= 2KK + 2 KM QM
@@ -198,34 +199,69 @@ __device__ __forceinline__ void set_status(int* status, int code) {
 // Small dense helpers on one CTA. Matrices are row-major with leading dim KM.
 // ---------------------------------------------------------------------------
 
-// C = A(mxk) * B(kxn); C must not alias A or B.
+// D += A B on an 8 x 8 tile, four columns of A at a time (FP64 tensor pipe): a
+// lane holds A[lane / 4][lane % 4], B[lane % 4][lane / 4] and
+// D[lane / 4][2 (lane % 4) + {0, 1}].
+__device__ __forceinline__ void w_mma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// The 8 x 8 blocks of an m x n result over the CTA's warps: f(r, j, o) with the
+// lane's row r of A, its column j of B (each possibly past the end, but inside
+// the padded tiles) and o, the first of the two columns of row r that its
+// accumulators hold. `rot` shifts the first block to another warp, so that
+// several small products in a row fill the warps.
+template <class F>
+__device__ __forceinline__ void for_blocks(int m, int n, int rot, F f) {
+    const int lane = threadIdx.x & 31, nb = (n + 7) >> 3, total = ((m + 7) >> 3) * nb;
+#pragma unroll 1
+    for (int b = ((int)(threadIdx.x >> 5) + NW - rot % NW) % NW; b < total; b += NW) {
+        const int rb = b / nb, jb = b - rb * nb;
+        f(8 * rb + (lane >> 2), 8 * jb + (lane >> 2), 8 * jb + 2 * (lane & 3));
+    }
+}
+
+// d += sum_{l < kd} a[l * sa] * b[l * sb], kd <= KM: `a` is the lane's row of A
+// and `b` its column of B. All operands are fetched before the first product:
+// the chain of products is what a block waits for, and a loop over l of unknown
+// length costs more than its six steps. Columns past kd count as zero.
+__device__ __forceinline__ void mma_dot(double (&d)[2], int kd, const double* a, int sa, const double* b, int sb) {
+    const int kr = threadIdx.x & 3;
+    double av[KM / 4], bv[KM / 4];
+#pragma unroll
+    for (int s = 0; s < KM / 4; ++s) {
+        const int l = 4 * s + kr;
+        av[s] = l < kd ? a[l * sa] : 0.0;
+        bv[s] = l < kd ? b[l * sb] : 0.0;
+    }
+#pragma unroll
+    for (int s = 0; s < KM / 4; s += 2)
+        if (4 * s < kd) {
+            w_mma(d, av[s], bv[s]);
+            w_mma(d, av[s + 1], bv[s + 1]);
+        }
+}
+
+// C = A(m x k) * B(k x n); C must not alias A or B.
 __device__ inline void sm_mm(double* C, const double* A, const double* B, int m, int k, int n) {
-    for (int e = threadIdx.x; e < m * n; e += NT) {
-        int i = e / n, j = e % n;
-        double s = 0.0;
-        for (int l = 0; l < k; ++l) s = fma(A[i * KM + l], B[l * KM + j], s);
-        C[i * KM + j] = s;
-    }
+    for_blocks(m, n, 0, [&](int r, int j, int o) {
+        double d[2] = {0.0, 0.0};
+        mma_dot(d, k, A + r * KM, 1, B + j, KM);
+        C[r * KM + o] = d[0];
+        C[r * KM + o + 1] = d[1];
+    });
     __syncthreads();
 }
-// C = A(mxk) * B^T (B is n x k)
+// C = A(m x k) * B^T (B is n x k)
 __device__ inline void sm_mmt(double* C, const double* A, const double* B, int m, int k, int n) {
-    for (int e = threadIdx.x; e < m * n; e += NT) {
-        int i = e / n, j = e % n;
-        double s = 0.0;
-        for (int l = 0; l < k; ++l) s = fma(A[i * KM + l], B[j * KM + l], s);
-        C[i * KM + j] = s;
-    }
-    __syncthreads();
-}
-// C = A^T(mxk, A is k x m) * B(kxn)
-__device__ inline void sm_tmm(double* C, const double* A, const double* B, int m, int k, int n) {
-    for (int e = threadIdx.x; e < m * n; e += NT) {
-        int i = e / n, j = e % n;
-        double s = 0.0;
-        for (int l = 0; l < k; ++l) s = fma(A[l * KM + i], B[l * KM + j], s);
-        C[i * KM + j] = s;
-    }
+    for_blocks(m, n, 0, [&](int r, int j, int o) {
+        double d[2] = {0.0, 0.0};
+        mma_dot(d, k, A + r * KM, 1, B + j * KM, 1);
+        C[r * KM + o] = d[0];
+        C[r * KM + o + 1] = d[1];
+    });
     __syncthreads();
 }
 __device__ inline void sm_copy(double* D, const double* A, int m, int n) {
@@ -359,88 +395,6 @@ static __device__ __noinline__ void jacobi_eig(double* Aw, double* V, double* la
     __syncthreads();
 }
 
-// Upper Cholesky R^T R = G (k x k, k <= KM <= 32) and Ri = R^{-1} by ONE warp:
-// lane c keeps column c of R and of R^{-1} in registers (fully unrolled loops,
-// so all register indices are static), row entries travel by shuffles.
-// Returns ||R||_F ||R^{-1}||_F, or +inf on breakdown (non-positive pivot).
-static __device__ __noinline__ double warp_chol_inv(const double* G, double* R, double* Ri, int k, int* bad_j = nullptr,
-                                double* bad_d = nullptr) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    double col[KM];
-    int first_bad = -1;
-    double first_d = 0.0;
-#pragma unroll
-    for (int a = 0; a < KM; ++a) col[a] = (lane < k && a < k && a <= lane) ? G[a * KM + lane] : 0.0;
-    bool ok = true;
-#pragma unroll
-    for (int j = 0; j < KM; ++j) {
-        if (j < k) {
-            double d = __shfl_sync(FULL, col[j], j);
-            if (!(d > 0.0)) {
-                if (ok) {
-                    first_bad = j;
-                    first_d = d;
-                }
-                ok = false;
-                d = 1.0;
-            }
-            const double piv = sqrt(d);
-            const double ip = 1.0 / piv;
-            if (lane == j) col[j] = piv;
-            else if (lane > j) col[j] *= ip;
-#pragma unroll
-            for (int a = j + 1; a < KM; ++a) {
-                if (a < k) {
-                    const double rja = __shfl_sync(FULL, col[j], a);
-                    if (lane >= a) col[a] = fma(-rja, col[j], col[a]);
-                }
-            }
-        }
-    }
-    // R to shared memory (column lane), then R^{-1} column lane by back substitution
-    if (lane < k) {
-#pragma unroll
-        for (int a = 0; a < KM; ++a)
-            if (a < k) R[a * KM + lane] = (a <= lane) ? col[a] : 0.0;
-    }
-    __syncwarp();
-    double inv[KM];
-    double nr = 0.0, ni = 0.0;
-#pragma unroll
-    for (int a = KM - 1; a >= 0; --a) {
-        double v = 0.0;
-        if (a < k && lane < k && a <= lane) {
-            double t = (a == lane) ? 1.0 : 0.0;
-#pragma unroll
-            for (int b = a + 1; b < KM; ++b)
-                if (b <= lane && b < k) t = fma(-R[a * KM + b], inv[b], t);
-            v = t / R[a * KM + a];
-        }
-        inv[a] = v;
-    }
-    if (lane < k) {
-#pragma unroll
-        for (int a = 0; a < KM; ++a)
-            if (a < k) {
-                Ri[a * KM + lane] = inv[a];
-                nr = fma(col[a], col[a], nr);
-                ni = fma(inv[a], inv[a], ni);
-            }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        nr += __shfl_xor_sync(FULL, nr, o);
-        ni += __shfl_xor_sync(FULL, ni, o);
-    }
-    ok = __all_sync(FULL, ok);
-    if (bad_j) *bad_j = first_bad;
-    if (bad_d) *bad_d = first_d;
-    return ok ? sqrt(nr) * sqrt(ni) : INFINITY;
-}
-
-// Two independent Cholesky factorisations on warps 0 and 1 concurrently
-// (either may be skipped). Writes the condition estimates; sets the status
-// flag on breakdown when `flag` is set.
 // On breakdown with `flag`, the first CTA to fail records in diag:
 // [0] stage tag, [1] side (0 = X, 1 = W), [2] k, [3] first bad pivot index,
 // [4] its value, [5] G[0][0], [6] min diagonal of G, [7] energy index.
@@ -460,44 +414,119 @@ __device__ inline void record_breakdown(double* diag, int* status, int tag, int 
     }
 }
 
-__device__ inline void dual_chol(bool dx, const double* GX, double* RX, double* RiX, int kx, double* condX,
-                          bool dw, const double* GW, double* RW, double* RiW, int kw, double* condW,
-                          int* status, bool flag, double* diag = nullptr, int tag = 0, int n = 0) {
-    __shared__ double s_c[2];
-    const int w = threadIdx.x >> 5;
-    if (w == 0 && dx) {
-        int bj;
-        double bd;
-        double c = warp_chol_inv(GX, RX, RiX, kx, &bj, &bd);
-        if ((threadIdx.x & 31) == 0) {
-            s_c[0] = c;
-            if (flag && !(c < INFINITY)) record_breakdown(diag, status, tag, 0, kx, bj, bd, GX, n);
-        }
-    }
-    if (w == 1 && dw) {
-        int bj;
-        double bd;
-        double c = warp_chol_inv(GW, RW, RiW, kw, &bj, &bd);
-        if ((threadIdx.x & 31) == 0) {
-            s_c[1] = c;
-            if (flag && !(c < INFINITY)) record_breakdown(diag, status, tag, 1, kw, bj, bd, GW, n);
-        }
+// Two upper Cholesky factorisations R^T R = G with R^{-1} side by side (either
+// may be skipped): the lower half of the CTA's warps takes X's, the upper half
+// W's. Elimination without square roots: the row operations that make
+// G = L D L^T upper triangular are applied to the identity as well (its rows grow
+// in the part of R below the diagonal), so that L^{-1} is there when the last
+// pivot is; R = D^{1/2} L^T and R^{-1} = L^{-T} D^{-1/2} are scaled at the end. The
+// chain of one step (pivot load, reciprocal, product, update, barrier) is what
+// bounds it. One warp per matrix, columns in registers and the inverse by back
+// substitution, took 25 us a pair at k = 20; this takes 8 us.
+// Writes the condition estimates ||R||_F ||R^{-1}||_F (+inf on a non-positive
+// pivot); `flag` makes a breakdown a device status.
+static __device__ __noinline__ void dual_chol(bool dx, const double* GX, double* RX, double* RiX, int kx, double* condX,
+                                              bool dw, const double* GW, double* RW, double* RiW, int kw, double* condW,
+                                              int* status, bool flag, double* diag = nullptr, int tag = 0, int n = 0) {
+    constexpr int HW = NW / 2, ROWS = (KM + HW - 1) / HW;
+    static_assert(KM <= 32, "one column of the matrix per lane");
+    __shared__ double s_nr[NW], s_ni[NW], s_d[2];
+    __shared__ int s_bad[2];
+    const int lane = threadIdx.x & 31, side = threadIdx.x >= NT / 2, warp = (threadIdx.x >> 5) - side * HW;
+    const bool on = side ? dw : dx;
+    const double* G = side ? GW : GX;
+    double* R = side ? RW : RX;
+    double* Ri = side ? RiW : RiX;
+    __builtin_assume(__isShared(G));
+    __builtin_assume(__isShared(R));
+    __builtin_assume(__isShared(Ri));
+    const int k = on ? (side ? kw : kx) : 0;
+    const int steps = max(dx ? kx : 0, dw ? kw : 0) - 1;
+    if (threadIdx.x < 2) s_bad[threadIdx.x] = -1;
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+        const int i = warp + u * HW;
+        if (i < k && lane < k) R[i * KM + lane] = lane >= i ? G[i * KM + lane] : 0.0;
     }
     __syncthreads();
-    if (condX) *condX = dx ? s_c[0] : 0.0;
-    if (condW) *condW = dw ? s_c[1] : 0.0;
-}
-
-// Row-wise triangular solve on a tile: Y[r,:] R = A[r,:] (R upper, k x k), in place.
-__device__ __forceinline__ void tile_rsolve(double* t, const double* R, const double* dinv_unused, int nr, int k) {
-    for (int r = threadIdx.x; r < nr; r += NT) {
-        double* row = t + r * KM;
-        for (int j = 0; j < k; ++j) {
-            double v = row[j];
-            for (int i = 0; i < j; ++i) v = fma(-row[i], R[i * KM + j], v);
-            row[j] = v / R[j * KM + j];
+    bool ok = true;
+    const auto pivot = [&](int j) {
+        const double d = R[j * KM + j];
+        if (ok && !(d > 0.0)) {
+            ok = false;
+            if (warp == 0 && lane == 0) {
+                s_bad[side] = j;
+                s_d[side] = d;
+            }
+        }
+        return d;
+    };
+#pragma unroll 1
+    for (int j = 0; j < steps; ++j) {
+        if (j < k - 1) {
+            const double d = pivot(j);
+            const double inv = -1.0 / (d > 0.0 ? d : 1.0);
+            const double rj = R[j * KM + min(lane, k - 1)];
+#pragma unroll
+            for (int u = 0; u < ROWS; ++u) {
+                const int i = j + 1 + warp + u * HW;
+                if (i < k) {
+                    const double f = R[j * KM + i] * inv;
+                    // columns l >= i: U; l < j: the identity's rows, whose entry j is f itself
+                    if (lane < k && (lane >= i || lane <= j))
+                        R[i * KM + lane] = lane == j ? f : fma(f, rj, R[i * KM + lane]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (k > 0) pivot(k - 1);
+    __syncthreads();
+    double nr = 0.0, ni = 0.0;
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+        const int i = warp + u * HW;
+        if (i < k) {
+            const double di = R[i * KM + i];
+            const double piv = di > 0.0 ? sqrt(di) : 1.0;
+            __syncwarp();
+            if (lane < k) {
+                const double v = lane == i ? piv : R[i * KM + lane] / piv;
+                const double w = lane == i ? 1.0 / piv : v;
+                R[i * KM + lane] = lane >= i ? v : 0.0;
+                Ri[lane * KM + i] = lane <= i ? w : 0.0;
+                nr = lane >= i ? fma(v, v, nr) : nr;
+                ni = lane <= i ? fma(w, w, ni) : ni;
+            }
         }
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        nr += __shfl_xor_sync(0xffffffffu, nr, o);
+        ni += __shfl_xor_sync(0xffffffffu, ni, o);
+    }
+    if (lane == 0) {
+        s_nr[side * HW + warp] = nr;
+        s_ni[side * HW + warp] = ni;
+    }
+    __syncthreads();
+    const auto cond = [&](int sd) -> double {
+        double tr = 0.0, ti = 0.0;
+#pragma unroll
+        for (int w = 0; w < HW; ++w) {
+            tr += s_nr[sd * HW + w];
+            ti += s_ni[sd * HW + w];
+        }
+        const double c = sqrt(tr) * sqrt(ti);
+        return s_bad[sd] < 0 && c < INFINITY ? c : INFINITY;
+    };
+    const double cx = dx ? cond(0) : 0.0, cw = dw ? cond(1) : 0.0;
+    if (flag && threadIdx.x == 0) {
+        if (!(cx < INFINITY)) record_breakdown(diag, status, tag, 0, kx, s_bad[0], s_bad[0] < 0 ? 0.0 : s_d[0], GX, n);
+        if (!(cw < INFINITY)) record_breakdown(diag, status, tag, 1, kw, s_bad[1], s_bad[1] < 0 ? 0.0 : s_d[1], GW, n);
+    }
+    __syncthreads();
+    if (condX) *condX = cx;
+    if (condW) *condW = cw;
 }
 
 }  // namespace titus

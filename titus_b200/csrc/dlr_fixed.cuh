@@ -12,28 +12,56 @@ __device__ __forceinline__ bool tsync(Ctx& x) {
 }
 
 // Publish this CTA's partial reduction of `count` entries and synchronise the
-// team. Large teams add a second stage: CTA b sums slice b of the entries over
-// all partials into the team's reduced buffer, then a second barrier; small
-// teams let every CTA sum the partials directly (reduce_into).
+// team; on return acc holds the team's sums. Large teams add a second stage:
+// CTA b sums slice b of the entries over all partials into the team's reduced
+// buffer, then a second barrier; small teams let every CTA sum the partials
+// directly. In the second stage a warp takes every NW-th partial and the warps'
+// sums are added in order: one thread per entry, walking all partials, waited
+// for G loads one after the other.
 __device__ inline bool publish_sync(Ctx& x, int count) {
+    __syncthreads();
     acc_publish(x, count);
     if (!tsync(x)) return false;
+    if (x.G == 1) return true;
     if (x.G <= kDirectReduceMax) {
-        x.red_mode = 0;
+        ProfScope ps(x.prof, PF_REDUCE);
+        for (int e = threadIdx.x; e < count; e += NT) {
+            double s = 0.0;
+#pragma unroll 4
+            for (int g = 0; g < x.G; ++g) s += ldcg(part_base(x, g) + e);
+            x.sm->acc[e] = s;
+        }
+        __syncthreads();
         return true;
     }
     {
         ProfScope ps(x.prof, PF_REDUCE);
-        const int per = (count + x.G - 1) / x.G;
+        static_assert(NW * 32 <= TR * KM, "the warps' sums lie in tile tA");
+        double* part = x.sm->tA;
+        const int per = (count + x.G - 1) / x.G, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const int e0 = x.b * per, e1 = min(count, e0 + per);
-        for (int e = e0 + threadIdx.x; e < e1; e += NT) {
-            double acc = 0.0;
-            for (int g = 0; g < x.G; ++g) acc += ldcg(part_base(x, g) + e);
-            x.st.red[e] = acc;
+        for (int eb = e0; eb < e1; eb += 32) {
+            double s = 0.0;
+            if (eb + lane < e1) {
+#pragma unroll 4
+                for (int g = warp; g < x.G; g += NW) s += ldcg(part_base(x, g) + eb + lane);
+            }
+            part[warp * 32 + lane] = s;
+            __syncthreads();
+            if (warp == 0 && eb + lane < e1) {
+                double t = part[lane];
+#pragma unroll
+                for (int w = 1; w < NW; ++w) t += part[w * 32 + lane];
+                x.st.red[eb + lane] = t;
+            }
+            __syncthreads();
         }
     }
-    x.red_mode = 1;
-    return tsync(x);
+    if (!tsync(x)) return false;
+    ProfScope ps(x.prof, PF_REDUCE);
+    for (int e = threadIdx.x; e < count; e += NT) x.sm->acc[e] = ldcg(x.st.red + e);
+    __syncthreads();
+    return true;
 }
 
 // ---- phase A: (pending) second dose half-step, boundary inflow, first dose
@@ -58,12 +86,25 @@ __device__ inline void phase_bc_dose(Ctx& x, int n, bool dose2_pending, bool do_
     const double* S = sm->slot[SL_S];
     double* v = sm->vec;  // S W[0,:]^T
     double* w0 = sm->vec + KM;
+    constexpr int LN = 4;             // lanes per cell: a cell's rows of X and psi are fetched in one go
+    constexpr int NX = KM / LN, NQ = 24 / LN;   // a handle takes at most 24 ordinates
+    const int ln = threadIdx.x % LN;
+    const auto sum4 = [](double a) {
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        return a + __shfl_xor_sync(0xffffffffu, a, 2);
+    };
     for (int j = threadIdx.x; j < k; j += NT) w0[j] = ldcg(x.st.W + j);
     __syncthreads();
-    for (int i = threadIdx.x; i < k; i += NT) {
+    if (threadIdx.x < KM * LN) {
+        const int i = threadIdx.x / LN;
         double s = 0.0;
-        for (int j = 0; j < k; ++j) s = fma(S[i * KM + j], w0[j], s);
-        v[i] = s;
+#pragma unroll
+        for (int u = 0; u < NX; ++u) {
+            const int j = ln + LN * u;
+            if (i < k && j < k) s = fma(S[i * KM + j], w0[j], s);
+        }
+        s = sum4(s);
+        if (ln == 0) v[i] = s;
     }
     __syncthreads();
     const double dE = P.dE;
@@ -71,30 +112,56 @@ __device__ inline void phase_bc_dose(Ctx& x, int n, bool dose2_pending, bool do_
     // half of step n-1 and the first half of step n (0-based index n-2)
     const double sd = P.stopping[n - 2];
     const double bce = P.bc_energy[n - 2];
-    for (int c = x.c0 + threadIdx.x; c < x.c1; c += NT) {
-        double xv = 0.0;
-        for (int j = 0; j < k; ++j) xv = fma(x.st.X[(size_t)c * KM + j], v[j], xv);
-        double* pr = x.psi_in + (size_t)c * QM;
-        double dose = x.st.dose[c];
+    for (int cb = x.c0; cb < x.c1; cb += NT / LN) {
+        const int c = cb + threadIdx.x / LN;
+        const bool on = c < x.c1;
+        const int cc = on ? c : x.c0;
+        double* xr = x.st.X + (size_t)cc * KM;
+        double* pr = x.psi_in + (size_t)cc * QM;
+        double xv = 0.0, xs[NX], ps[NQ], m[NQ];
+#pragma unroll
+        for (int u = 0; u < NX; ++u) xs[u] = ln + LN * u < k ? xr[ln + LN * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < NQ; ++u) {
+            const bool in = ln + LN * u < P.q;
+            ps[u] = in ? pr[ln + LN * u] : 0.0;
+            m[u] = in ? P.mred[ln + LN * u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < NX; ++u)
+            if (ln + LN * u < k) xv = fma(xs[u], v[ln + LN * u], xv);
+        xv = sum4(xv);
+        double dose = x.st.dose[cc];
         if (dose2_pending) {
             double u = 0.0;
-            for (int kq = 0; kq < P.q; ++kq) u = fma(pr[kq], P.mred[kq], u);
-            dose += 0.5 * dE * (xv + u) * sd * P.rinv[c];
+#pragma unroll
+            for (int h = 0; h < NQ; ++h) u = fma(ps[h], m[h], u);
+            u = sum4(u);
+            dose += 0.5 * dE * (xv + u) * sd * P.rinv[cc];
         }
-        bool bnd = is_bnd(P, c);
+        const bool bnd = is_bnd(P, cc);
         if (do_bc) {
-            const int src = two_layer ? bc2_source(P, c) : (bnd ? c : -1);
+            const int src = two_layer ? bc2_source(P, cc) : (bnd ? cc : -1);
             if (src >= 0) {
-                double bs = bce * P.bc_space[src];
-                for (int kq = 0; kq < P.q; ++kq) pr[kq] = bs * P.bc_angle[kq];
+                const double bs = bce * P.bc_space[src];
+#pragma unroll
+                for (int h = 0; h < NQ; ++h)
+                    if (ln + LN * h < P.q) {
+                        ps[h] = bs * P.bc_angle[ln + LN * h];
+                        if (on) pr[ln + LN * h] = ps[h];
+                    }
             }
             double u = 0.0;
-            for (int kq = 0; kq < P.q; ++kq) u = fma(pr[kq], P.mred[kq], u);
-            dose += 0.5 * dE * (xv + u) * sd * P.rinv[c];
-            if (bnd)
-                for (int j = 0; j < k; ++j) x.st.X[(size_t)c * KM + j] = 0.0;
+#pragma unroll
+            for (int h = 0; h < NQ; ++h) u = fma(ps[h], m[h], u);
+            u = sum4(u);
+            dose += 0.5 * dE * (xv + u) * sd * P.rinv[cc];
+            if (bnd && on)
+#pragma unroll
+                for (int h = 0; h < NX; ++h)
+                    if (ln + LN * h < k) xr[ln + LN * h] = 0.0;
         }
-        x.st.dose[c] = dose;
+        if (on && ln == 0) x.st.dose[c] = dose;
     }
 }
 
@@ -151,72 +218,40 @@ __device__ inline void sweep_cells(Ctx& x, double sigma0, bool limited = false) 
 // L2x/Ax, L2y/Az, L1x/|Ax|, L1y/|Az|; nops = 2: the central pair only.
 __device__ inline void stream_grams_partial(Ctx& x, int nops = 4) {
     SmemLayout* sm = x.sm;
-    const int k = x.k;
-    for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-        int nr = min(TR, x.c1 - r0);
-        load_rows(sm->tA, x.st.X, r0, nr, k);
-        if (nops == 2) stencil2_tile(x, x.st.X, r0, nr, k, sm->tL);
-        else stencil_tile(x, x.st.X, r0, nr, k, sm->tL);
+    const int k = x.k, tr = tile_rows(x.c1 - x.c0), tw = tile_rows(x.m1 - x.m0), per = ((k + 7) >> 3) * ((k + 7) >> 3);
+    for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+        int nr = min(tr, x.c1 - r0);
+        stencil_tile(x, x.st.X, r0, nr, k, sm->tL, sm->tA, nops == 2);
         __syncthreads();
-        for (int d = 0; d < nops; ++d) gram_acc(sm->acc, d * k * k, sm->tA, KM, k, sm->tL[d], KM, k, nr);
+        for (int d = 0; d < nops; ++d) gram_acc(sm->acc, d * k * k, sm->tA, KM, k, sm->tL[d], KM, k, nr, d * per);
         __syncthreads();
     }
-    for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-        int nr = min(TR, x.m1 - r0);
+    for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+        int nr = min(tw, x.m1 - r0);
         load_rows(sm->tA, x.st.W, r0, nr, k);
         spmm_tile(x, x.st.W, r0, nr, k, sm->tL, nops);
         __syncthreads();
-        for (int d = 0; d < nops; ++d) gram_acc(sm->acc, (nops + d) * k * k, sm->tA, KM, k, sm->tL[d], KM, k, nr);
+        for (int d = 0; d < nops; ++d)
+            gram_acc(sm->acc, (nops + d) * k * k, sm->tA, KM, k, sm->tL[d], KM, k, nr, d * per);
         __syncthreads();
     }
 }
 
-// ---- range finder pass 1 (G1 = (A V)^T (A V)) on one side; A is n x k in global
-__device__ inline void rf_pass_b(Ctx& x, const double* A, int r0b, int r1b, const double* V, int k, int off) {
+// ---- range finder passes on one side: Y = A M (A is n x k in global, M is
+// k x w), G = Y^T Y, and Y to Cbuf unless it is null.
+__device__ inline void rf_pass(Ctx& x, const double* A, double* Cbuf, int r0b, int r1b, const double* M, int k, int w,
+                               int off) {
     SmemLayout* sm = x.sm;
-    for (int r0 = r0b; r0 < r1b; r0 += TR) {
-        int nr = min(TR, r1b - r0);
+    const int tr = tile_rows(r1b - r0b);
+    for (int r0 = r0b; r0 < r1b; r0 += tr) {
+        int nr = min(tr, r1b - r0);
         load_rows(sm->tA, A, r0, nr, k);
         __syncthreads();
-        tile_mm(sm->tO, sm->tA, V, nr, k, k);
+        tile_mm(sm->tO, sm->tA, M, nr, k, w, Cbuf, r0);
         __syncthreads();
-        gram_acc(sm->acc, off, sm->tO, KM, k, sm->tO, KM, k, nr);
-        __syncthreads();
+        gram_acc(sm->acc, off, sm->tO, KM, w, sm->tO, KM, w, nr);
     }
-}
-// ---- range finder pass 2: C = A T1 (written to Cbuf), G2 = C^T C
-__device__ inline void rf_pass_c(Ctx& x, const double* A, double* Cbuf, int r0b, int r1b, const double* T1, int k,
-                          int rho, int off) {
-    SmemLayout* sm = x.sm;
-    for (int r0 = r0b; r0 < r1b; r0 += TR) {
-        int nr = min(TR, r1b - r0);
-        load_rows(sm->tA, A, r0, nr, k);
-        __syncthreads();
-        tile_mm(sm->tO, sm->tA, T1, nr, k, rho);
-        __syncthreads();
-        store_rows(Cbuf, sm->tO, r0, nr, rho);
-        gram_acc(sm->acc, off, sm->tO, KM, rho, sm->tO, KM, rho, nr);
-        __syncthreads();
-    }
-}
-
-// Range-finder pass of the fast path: Y = A R^{-1} by row-wise triangular
-// solves (written to Cbuf), G = Y^T Y.
-// Rows are processed in chunks of kBigRows over the contiguous tile area
-// tA..tO (free during the range finder), one thread per row for the solve.
-__device__ inline void rf_pass_solve(Ctx& x, const double* A, double* Cbuf, int r0b, int r1b, const double* R, int k, int off) {
-    SmemLayout* sm = x.sm;
-    double* big = sm->tA;
-    for (int r0 = r0b; r0 < r1b; r0 += kBigRows) {
-        int nr = min(kBigRows, r1b - r0);
-        load_rows(big, A, r0, nr, k);
-        __syncthreads();
-        tile_rsolve(big, R, nullptr, nr, k);
-        __syncthreads();
-        store_rows(Cbuf, big, r0, nr, k);
-        gram_acc(sm->acc, off, big, KM, k, big, KM, k, nr);
-        __syncthreads();
-    }
+    __syncthreads();
 }
 
 // Orthonormal bases of the numerical ranges of A_X (own cells) and A_W (own
@@ -225,7 +260,7 @@ __device__ inline void rf_pass_solve(Ctx& x, const double* A, double* Cbuf, int 
 // slots SL_RIK/SL_RIL the inverse R of its CholQR, so that the basis is
 // C R^{-1} (rho columns) followed by the completion vectors.
 //  fast path: Cholesky of G0 with ||R||_F ||R^-1||_F < 1e5 certifies full
-//    numerical rank; C = A R0^{-1} (row solves), then CholQR of C.
+//    numerical rank; C = A R0^{-1}, then CholQR of C.
 //  rank-revealing path: Jacobi eig of G0 -> V; Gram of A V -> Jacobi -> V2,
 //    nu; C = A V V2_J / nu_J with nu_j > tol nu_0; CholQR of C.
 // Returns false if the team aborted.
@@ -256,12 +291,12 @@ static __device__ __noinline__ bool range_finder(Ctx& x, const double* AX, const
         ProfScope ps(x.prof, PF_RF_PASSES);
         acc_zero(x, 2 * k * k);
         if (doX) {
-            if (fastX) rf_pass_solve(x, AX, x.CX, x.c0, x.c1, sm->slot[SL_RK], k, 0);
-            else rf_pass_b(x, AX, x.c0, x.c1, sm->slot[SL_VK], k, 0);
+            if (fastX) rf_pass(x, AX, x.CX, x.c0, x.c1, sm->slot[SL_RIK], k, k, 0);
+            else rf_pass(x, AX, nullptr, x.c0, x.c1, sm->slot[SL_VK], k, k, 0);
         }
         if (doW) {
-            if (fastW) rf_pass_solve(x, AW, x.CW, x.m0, x.m1, sm->slot[SL_RL], k, k * k);
-            else rf_pass_b(x, AW, x.m0, x.m1, sm->slot[SL_VL], k, k * k);
+            if (fastW) rf_pass(x, AW, x.CW, x.m0, x.m1, sm->slot[SL_RIL], k, k, k * k);
+            else rf_pass(x, AW, nullptr, x.m0, x.m1, sm->slot[SL_VL], k, k, k * k);
         }
     }
     if (!publish_sync(x, 2 * k * k)) return false;
@@ -286,8 +321,8 @@ static __device__ __noinline__ bool range_finder(Ctx& x, const double* AX, const
         {
             ProfScope ps(x.prof, PF_RF_PASSES);
             acc_zero(x, 2 * k * k);
-            if (slowX) rf_pass_c(x, AX, x.CX, x.c0, x.c1, sm->slot[SL_TK], k, x.rhoK, 0);
-            if (slowW) rf_pass_c(x, AW, x.CW, x.m0, x.m1, sm->slot[SL_TL], k, x.rhoL, k * k);
+            if (slowX) rf_pass(x, AX, x.CX, x.c0, x.c1, sm->slot[SL_TK], k, x.rhoK, 0);
+            if (slowW) rf_pass(x, AW, x.CW, x.m0, x.m1, sm->slot[SL_TL], k, x.rhoL, k * k);
         }
         if (!publish_sync(x, 2 * k * k)) return false;
         if (slowX) reduce_into(x, 0, x.rhoK, x.rhoK, sm->ja);
@@ -311,6 +346,27 @@ static __device__ __noinline__ bool range_finder(Ctx& x, const double* AX, const
 __device__ inline void sm_asbt(double* D, const double* A, const double* S, const double* B, double* tmp, int k) {
     sm_mm(tmp, A, S, k, k, k);
     sm_mmt(D, tmp, B, k, k, k);
+}
+
+// small: D = A^T B^T (k x k); D aliases neither
+__device__ inline void sm_stgt(double* D, const double* A, const double* B, int k) {
+    for_blocks(k, k, 0, [&](int r, int j, int o) {
+        double d[2] = {0.0, 0.0};
+        mma_dot(d, k, A + r, KM, B + j * KM, 1);
+        D[r * KM + o] = d[0];
+        D[r * KM + o + 1] = d[1];
+    });
+    __syncthreads();
+}
+
+// rows [r0, r0+nr) of MRed into tile tP, times the moments' cross-sections if given
+__device__ inline void load_mred(Ctx& x, int r0, int nr, const double* sig) {
+    const DevProblem& P = x.P;
+    for (int e = threadIdx.x; e < nr * P.q; e += NT) {
+        const int r = e / P.q, kq = e - r * P.q;
+        const double v = P.mred[(size_t)r0 * P.q + e];
+        x.sm->tP[r * QM + kq] = sig ? v * sig[P.lof[r0 + r]] : v;
+    }
 }
 
 // ---- RK4 streaming of K and L (SolverCSD.jl:724-758), the RK4 ("HighOrder")
@@ -352,85 +408,82 @@ static __device__ __noinline__ bool rk4_stream(Ctx& x) {
         if (s == 4) acc_zero(x, 2 * k * k);
         {
             ProfScope ps(x.prof, PF_ROWS_STREAM);
-            for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-                const int nr = min(TR, x.c1 - r0);
-                if (s == 1) {
-                    load_rows(sm->tA, x.st.X, r0, nr, k);
-                    stencil2_tile(x, x.st.X, r0, nr, k, sm->tL);
-                } else {
-                    stencil2_tile(x, Yin, r0, nr, k, sm->tL);
-                }
+            const int tr = tile_rows(x.c1 - x.c0), tw = tile_rows(x.m1 - x.m0);
+            for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+                const int nr = min(tr, x.c1 - r0);
+                stencil_tile(x, s == 1 ? x.st.X : Yin, r0, nr, k, sm->tL, s == 1 ? sm->tA : nullptr, true);
                 __syncthreads();
-                for (int e = threadIdx.x; e < nr * k; e += NT) {
-                    const int r = e / k, j = e - (e / k) * k;
-                    const size_t g = (size_t)(r0 + r) * KM + j;
-                    double t = 0.0;
-                    for (int l = 0; l < k; ++l) t = fma(sm->tL[0][r * KM + l], C0[l * KM + j], t);
-                    for (int l = 0; l < k; ++l) t = fma(sm->tL[1][r * KM + l], C1[l * KM + j], t);
-                    const double kd = -t;
-                    double Kv;
-                    if (s == 1) {
-                        Kv = 0.0;
-                        for (int l = 0; l < k; ++l) Kv = fma(sm->tA[r * KM + l], Sm[l * KM + j], Kv);
-                        x.st.K[g] = Kv;
-                        KUP[g] = Kv + dE * kd / 6;
-                    } else {
-                        Kv = ldcg(x.st.K + g);
-                        if (s < 4) KUP[g] = ldcg(KUP + g) + wup * dE * kd / 6;
+                for_blocks(nr, k, 0, [&](int r, int jb, int o) {
+                    double t[2] = {0.0, 0.0}, kv[2] = {0.0, 0.0};
+                    mma_dot(t, k, sm->tL[0] + r * KM, 1, C0 + jb, KM);
+                    mma_dot(t, k, sm->tL[1] + r * KM, 1, C1 + jb, KM);
+                    if (s == 1) mma_dot(kv, k, sm->tA + r * KM, 1, Sm + jb, KM);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int j = o + h;
+                        if (r >= nr || j >= k) continue;
+                        const size_t g = (size_t)(r0 + r) * KM + j;
+                        const double kd = -t[h];
+                        double Kv;
+                        if (s == 1) {
+                            Kv = kv[h];
+                            x.st.K[g] = Kv;
+                            KUP[g] = Kv + dE * kd / 6;
+                        } else {
+                            Kv = ldcg(x.st.K + g);
+                            if (s < 4) KUP[g] = ldcg(KUP + g) + wup * dE * kd / 6;
+                        }
+                        if (s < 4) {
+                            Yout[g] = Kv + cnext * kd;
+                        } else {
+                            const double Kn = ldcg(KUP + g) + dE * kd / 6;
+                            sm->tO[r * KM + j] = Kn;
+                            x.st.K[g] = Kn;
+                        }
                     }
-                    if (s < 4) {
-                        Yout[g] = Kv + cnext * kd;
-                    } else {
-                        const double Kn = ldcg(KUP + g) + dE * kd / 6;
-                        sm->tO[r * KM + j] = Kn;
-                    }
-                }
+                });
                 __syncthreads();
-                if (s == 4) {
-                    store_rows(x.st.K, sm->tO, r0, nr, k);
-                    gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tO, KM, k, nr);
-                    __syncthreads();
-                }
+                if (s == 4) gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tO, KM, k, nr);
             }
-            for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-                const int nr = min(TR, x.m1 - r0);
-                if (s == 1) {
-                    load_rows(sm->tA, x.st.W, r0, nr, k);
-                    spmm_tile(x, x.st.W, r0, nr, k, sm->tL, 2);
-                } else {
-                    spmm_tile(x, Lin, r0, nr, k, sm->tL, 2);
-                }
+            __syncthreads();
+            for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+                const int nr = min(tw, x.m1 - r0);
+                if (s == 1) load_rows(sm->tA, x.st.W, r0, nr, k);
+                spmm_tile(x, s == 1 ? x.st.W : Lin, r0, nr, k, sm->tL, 2);
                 __syncthreads();
-                for (int e = threadIdx.x; e < nr * k; e += NT) {
-                    const int r = e / k, j = e - (e / k) * k;
-                    const size_t g = (size_t)(r0 + r) * KM + j;
-                    double t = 0.0;
-                    for (int l = 0; l < k; ++l) t = fma(sm->tL[0][r * KM + l], H0[l * KM + j], t);
-                    for (int l = 0; l < k; ++l) t = fma(sm->tL[1][r * KM + l], H1[l * KM + j], t);
-                    const double ld = -t;
-                    double Lv;
-                    if (s == 1) {
-                        Lv = 0.0;  // (W S^T)[r][j]
-                        for (int l = 0; l < k; ++l) Lv = fma(sm->tA[r * KM + l], Sm[j * KM + l], Lv);
-                        x.st.L[g] = Lv;
-                        LUP[g] = ld;
-                    } else {
-                        Lv = ldcg(x.st.L + g);
-                        if (s < 4) LUP[g] = ldcg(LUP + g) + wup * ld;
+                for_blocks(nr, k, 0, [&](int r, int jb, int o) {
+                    double t[2] = {0.0, 0.0}, lv[2] = {0.0, 0.0};
+                    mma_dot(t, k, sm->tL[0] + r * KM, 1, H0 + jb, KM);
+                    mma_dot(t, k, sm->tL[1] + r * KM, 1, H1 + jb, KM);
+                    if (s == 1) mma_dot(lv, k, sm->tA + r * KM, 1, Sm + jb * KM, 1);   // (W S^T)[r][j]
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int j = o + h;
+                        if (r >= nr || j >= k) continue;
+                        const size_t g = (size_t)(r0 + r) * KM + j;
+                        const double ld = -t[h];
+                        double Lv;
+                        if (s == 1) {
+                            Lv = lv[h];
+                            x.st.L[g] = Lv;
+                            LUP[g] = ld;
+                        } else {
+                            Lv = ldcg(x.st.L + g);
+                            if (s < 4) LUP[g] = ldcg(LUP + g) + wup * ld;
+                        }
+                        if (s < 4) {
+                            Lout[g] = Lv + cnext * ld;
+                        } else {
+                            const double Ln = Lv + dE * (ldcg(LUP + g) + ld) / 6;
+                            sm->tO[r * KM + j] = Ln;
+                            x.st.L[g] = Ln;
+                        }
                     }
-                    if (s < 4) {
-                        Lout[g] = Lv + cnext * ld;
-                    } else {
-                        sm->tO[r * KM + j] = Lv + dE * (ldcg(LUP + g) + ld) / 6;
-                    }
-                }
+                });
                 __syncthreads();
-                if (s == 4) {
-                    store_rows(x.st.L, sm->tO, r0, nr, k);
-                    gram_acc(sm->acc, k * k, sm->tO, KM, k, sm->tO, KM, k, nr);
-                    __syncthreads();
-                }
+                if (s == 4) gram_acc(sm->acc, k * k, sm->tO, KM, k, sm->tO, KM, k, nr);
             }
+            __syncthreads();
         }
         if (s < 4) {
             if (!tsync(x)) return false;
@@ -500,7 +553,6 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
     x.st = states[blockIdx.x / G];
     x.sm = sm;
     x.prof = (blockIdx.x == 0) ? P.prof : nullptr;
-    x.red_mode = 0;
     x.gen = 0;
     x.parity = 0;
     x.rhoK = x.rhoL = 0;
@@ -522,6 +574,7 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
     int steps = 0;
     constexpr bool HO = (METHOD == kHighOrder);   // RK4 integrator (SolveFirstCollisionSourceDLRHighOrder)
     constexpr int nops = HO ? 2 : 4;               // streaming operators: central pair, or with Roe terms
+    const int tr = tile_rows(x.c1 - x.c0), tw = tile_rows(x.m1 - x.m0);
     double* Sm = sm->slot[SL_S];
     for (int n = n_begin; n <= n_end; ++n) {
         x.psi_in = psi_idx ? x.st.psi1 : x.st.psi0;
@@ -554,11 +607,8 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
                 for (int e = threadIdx.x; e < k * k; e += NT) {
                     int i = e / k, j = e % k;
                     sm->slot[SL_G0 + d][i * KM + j] = sm->slot[SL_P0][j * KM + i];
-                    double s2 = 0.0;
-                    for (int l = 0; l < k; ++l) s2 = fma(Sm[l * KM + i], sm->slot[SL_P0][j * KM + l], s2);
-                    sm->slot[SL_G0 + 2 + d][i * KM + j] = s2;
                 }
-                __syncthreads();
+                sm_stgt(sm->slot[SL_G0 + 2 + d], Sm, sm->slot[SL_P0], k);
             }
             // ---------------- phase C (RK4): K and L streaming updates
             if (!rk4_stream(x)) return;
@@ -571,56 +621,45 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
             // SC_d = S C_d -> slot C_d ; SG_d = S^T G_d^T -> slot G_d
             for (int d = 0; d < 4; ++d) {
                 sm_mm(sm->slot[SL_P0], Sm, sm->slot[SL_C0 + d], k, k, k);
+                sm_stgt(sm->slot[SL_P0 + 1], Sm, sm->slot[SL_G0 + d], k);
                 sm_copy(sm->slot[SL_C0 + d], sm->slot[SL_P0], k, k);
-                // (S^T G^T)[i][j] = sum_l S[l][i] G[j][l]
-                for (int e = threadIdx.x; e < k * k; e += NT) {
-                    int i = e / k, j = e % k;
-                    double s = 0.0;
-                    for (int l = 0; l < k; ++l) s = fma(Sm[l * KM + i], sm->slot[SL_G0 + d][j * KM + l], s);
-                    sm->slot[SL_P0][i * KM + j] = s;
-                }
-                __syncthreads();
-                sm_copy(sm->slot[SL_G0 + d], sm->slot[SL_P0], k, k);
+                sm_copy(sm->slot[SL_G0 + d], sm->slot[SL_P0 + 1], k, k);
             }
             // ---------------- phase C: K and L streaming updates
             acc_zero(x, 2 * k * k);
-            for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-                int nr = min(TR, x.c1 - r0);
-                load_rows(sm->tA, x.st.X, r0, nr, k);
-                stencil_tile(x, x.st.X, r0, nr, k, sm->tL);
+            for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+                const int nr = min(tr, x.c1 - r0);
+                stencil_tile(x, x.st.X, r0, nr, k, sm->tL, sm->tA, false);
                 __syncthreads();
-                for (int e = threadIdx.x; e < nr * k; e += NT) {
-                    int r = e / k, j = e % k;
-                    double s = 0.0;
-                    for (int l = 0; l < k; ++l) s = fma(sm->tA[r * KM + l], Sm[l * KM + j], s);
-                    double t = 0.0;
-                    for (int d = 0; d < 4; ++d)
-                        for (int l = 0; l < k; ++l) t = fma(sm->tL[d][r * KM + l], sm->slot[SL_C0 + d][l * KM + j], t);
-                    sm->tO[r * KM + j] = s - dE * t;
-                }
+                for_blocks(nr, k, 0, [&](int r, int j, int o) {
+                    double a[2] = {0.0, 0.0}, t[2] = {0.0, 0.0};
+                    mma_dot(a, k, sm->tA + r * KM, 1, Sm + j, KM);
+#pragma unroll
+                    for (int d = 0; d < 4; ++d) mma_dot(t, k, sm->tL[d] + r * KM, 1, sm->slot[SL_C0 + d] + j, KM);
+                    if (r < nr)
+                        put_pair(sm->tO + r * KM, x.st.K + (size_t)(r0 + r) * KM, k, o, a[0] - dE * t[0],
+                                 a[1] - dE * t[1]);
+                });
                 __syncthreads();
-                store_rows(x.st.K, sm->tO, r0, nr, k);
                 gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tO, KM, k, nr);
-                __syncthreads();
             }
-            for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-                int nr = min(TR, x.m1 - r0);
+            __syncthreads();
+            for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+                const int nr = min(tw, x.m1 - r0);
                 load_rows(sm->tA, x.st.W, r0, nr, k);
                 spmm_tile(x, x.st.W, r0, nr, k, sm->tL);
                 __syncthreads();
-                for (int e = threadIdx.x; e < nr * k; e += NT) {
-                    int r = e / k, j = e % k;
-                    double s = 0.0;  // (W S^T)[r][j] = sum_l W[r][l] S[j][l]
-                    for (int l = 0; l < k; ++l) s = fma(sm->tA[r * KM + l], Sm[j * KM + l], s);
-                    double t = 0.0;
-                    for (int d = 0; d < 4; ++d)
-                        for (int l = 0; l < k; ++l) t = fma(sm->tL[d][r * KM + l], sm->slot[SL_G0 + d][l * KM + j], t);
-                    sm->tO[r * KM + j] = s - dE * t;
-                }
+                for_blocks(nr, k, 0, [&](int r, int j, int o) {
+                    double a[2] = {0.0, 0.0}, t[2] = {0.0, 0.0};
+                    mma_dot(a, k, sm->tA + r * KM, 1, Sm + j * KM, 1);   // (W S^T)[r][j]
+#pragma unroll
+                    for (int d = 0; d < 4; ++d) mma_dot(t, k, sm->tL[d] + r * KM, 1, sm->slot[SL_G0 + d] + j, KM);
+                    if (r < nr)
+                        put_pair(sm->tO + r * KM, x.st.L + (size_t)(r0 + r) * KM, k, o, a[0] - dE * t[0],
+                                 a[1] - dE * t[1]);
+                });
                 __syncthreads();
-                store_rows(x.st.L, sm->tO, r0, nr, k);
                 gram_acc(sm->acc, k * k, sm->tO, KM, k, sm->tO, KM, k, nr);
-                __syncthreads();
             }
             if (!publish_sync(x, 2 * k * k)) return;
         }
@@ -629,24 +668,16 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
             if (!range_finder(x, x.st.K, x.st.L, true, true, k)) return;
             // ---------------- phase F: new bases, MUp = XNew^T X, NUp = WNew^T W
             acc_zero(x, 2 * k * k);
-            for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-                int nr = min(TR, x.c1 - r0);
-                x_basis_tile(x, r0, nr, x.rhoK, k, sm->tO);
-                load_rows(sm->tA, x.st.X, r0, nr, k);
-                __syncthreads();
-                gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tA, KM, k, nr);
-                __syncthreads();
-                store_rows(x.st.X, sm->tO, r0, nr, k);
+            for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+                const int nr = min(tr, x.c1 - r0);
+                x_basis_tile(x, r0, nr, x.rhoK, k, sm->tO, sm->tL[0]);
+                gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tL[0], KM, k, nr);
                 __syncthreads();
             }
-            for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-                int nr = min(TR, x.m1 - r0);
-                w_basis_tile(x, r0, nr, x.rhoL, k - x.rhoL, sm->tO);
-                load_rows(sm->tA, x.st.W, r0, nr, k);
-                __syncthreads();
-                gram_acc(sm->acc, k * k, sm->tO, KM, k, sm->tA, KM, k, nr);
-                __syncthreads();
-                store_rows(x.st.W, sm->tO, r0, nr, k);
+            for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+                const int nr = min(tw, x.m1 - r0);
+                w_basis_tile(x, r0, nr, x.rhoL, k - x.rhoL, sm->tO, x.st.W, sm->tL[0], k);
+                gram_acc(sm->acc, k * k, sm->tO, KM, k, sm->tL[0], KM, k, nr);
                 __syncthreads();
             }
             if (!publish_sync(x, 2 * k * k)) return;
@@ -690,28 +721,26 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
             if (is_bnd(P, c))
                 for (int j = 0; j < k; ++j) x.st.X[(size_t)c * KM + j] = 0.0;
         __syncthreads();
-        for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-            int nr = min(TR, x.m1 - r0);
+        for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+            const int nr = min(tw, x.m1 - r0);
             load_rows(sm->tA, x.st.W, r0, nr, k);
             __syncthreads();
-            for (int e = threadIdx.x; e < nr * k; e += NT) {
-                int r = e / k, j = e % k;
-                double s = 0.0;
-                for (int l = 0; l < k; ++l) s = fma(sm->tA[r * KM + l], Sm[j * KM + l], s);
-                int m = r0 + r;
-                double D = sig[0] - sig[P.lof[m]];
-                sm->tO[r * KM + j] = s / (1.0 + dE * D);
-            }
+            for_blocks(nr, k, 0, [&](int r, int j, int o) {
+                double a[2] = {0.0, 0.0};
+                mma_dot(a, k, sm->tA + r * KM, 1, Sm + j * KM, 1);
+                if (r < nr) {
+                    const double den = 1.0 + dE * (sig[0] - sig[P.lof[r0 + r]]);
+                    put_pair(sm->tO + r * KM, x.st.L + (size_t)(r0 + r) * KM, k, o, a[0] / den, a[1] / den);
+                }
+            });
             __syncthreads();
-            store_rows(x.st.L, sm->tO, r0, nr, k);
             gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tO, KM, k, nr);
-            __syncthreads();
         }
-        for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-            int nr = min(TR, x.c1 - r0);
+        __syncthreads();
+        for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+            const int nr = min(tr, x.c1 - r0);
             load_rows(sm->tA, x.st.X, r0, nr, k);
-            for (int e = threadIdx.x; e < nr * P.q; e += NT)
-                sm->tP[(e / P.q) * QM + e % P.q] = ldcg(x.psi_in + (size_t)(r0 + e / P.q) * QM + e % P.q);
+            load_rows(sm->tP, x.psi_in, r0, nr, P.q, QM);
             __syncthreads();
             gram_acc(sm->acc, k * k, sm->tP, QM, P.q, sm->tA, KM, k, nr);
             __syncthreads();
@@ -723,20 +752,12 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
         if (!range_finder(x, nullptr, x.st.L, false, true, k)) return;
         // ---------------- phase K: W = basis(L); S = L^T W ; Bk = MRed^T diag(Dvec) W
         acc_zero(x, k * k + P.q * k);
-        for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-            int nr = min(TR, x.m1 - r0);
-            w_basis_tile(x, r0, nr, x.rhoL, k - x.rhoL, sm->tO);
-            load_rows(sm->tA, x.st.L, r0, nr, k);
-            for (int e = threadIdx.x; e < nr * P.q; e += NT) {
-                int r = e / P.q, kq = e % P.q;
-                int m = r0 + r;
-                sm->tP[r * QM + kq] = P.mred[(size_t)m * P.q + kq] * sig[P.lof[m]];
-            }
-            __syncthreads();
-            gram_acc(sm->acc, 0, sm->tA, KM, k, sm->tO, KM, k, nr);
-            gram_acc(sm->acc, k * k, sm->tP, QM, P.q, sm->tO, KM, k, nr);
-            __syncthreads();
-            store_rows(x.st.W, sm->tO, r0, nr, k);
+        for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+            const int nr = min(tw, x.m1 - r0);
+            load_mred(x, r0, nr, sig);
+            w_basis_tile(x, r0, nr, x.rhoL, k - x.rhoL, sm->tO, x.st.L, sm->tL[0], k);
+            gram_acc(sm->acc, 0, sm->tL[0], KM, k, sm->tO, KM, k, nr);
+            gram_acc(sm->acc, k * k, sm->tP, QM, P.q, sm->tO, KM, k, nr, NW / 2);
             __syncthreads();
         }
         if (!publish_sync(x, k * k + P.q * k)) return;
@@ -744,78 +765,61 @@ dlr_kernel(DevProblem P, TeamState* states, int G, int n_begin, int n_end, int d
         reduce_into(x, k * k, P.q, k, sm->slot[SL_P0 + 2]);  // Bk (q x k)
         // ---------------- phase L: in-scattering K (X side) and L (W side)
         acc_zero(x, 2 * k * k);
-        for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-            int nr = min(TR, x.c1 - r0);
+        for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+            const int nr = min(tr, x.c1 - r0);
             load_rows(sm->tA, x.st.X, r0, nr, k);
-            for (int e = threadIdx.x; e < nr * P.q; e += NT)
-                sm->tP[(e / P.q) * QM + e % P.q] = ldcg(x.psi_in + (size_t)(r0 + e / P.q) * QM + e % P.q);
+            load_rows(sm->tP, x.psi_in, r0, nr, P.q, QM);
             __syncthreads();
-            for (int e = threadIdx.x; e < nr * k; e += NT) {
-                int r = e / k, j = e % k;
-                double s = 0.0;
-                if (!is_bnd(P, r0 + r)) {
-                    for (int l = 0; l < k; ++l) s = fma(sm->tA[r * KM + l], Sm[l * KM + j], s);
-                    double t = 0.0;
-                    for (int kq = 0; kq < P.q; ++kq) t = fma(sm->tP[r * QM + kq], sm->slot[SL_P0 + 2][kq * KM + j], t);
-                    s += dE * t;
+            for_blocks(nr, k, 0, [&](int r, int j, int o) {
+                double a[2] = {0.0, 0.0}, t[2] = {0.0, 0.0};
+                mma_dot(a, k, sm->tA + r * KM, 1, Sm + j, KM);
+                mma_dot(t, P.q, sm->tP + r * QM, 1, sm->slot[SL_P0 + 2] + j, KM);
+                if (r < nr) {
+                    const bool bnd = is_bnd(P, r0 + r);
+                    put_pair(sm->tO + r * KM, x.st.K + (size_t)(r0 + r) * KM, k, o, bnd ? 0.0 : a[0] + dE * t[0],
+                             bnd ? 0.0 : a[1] + dE * t[1]);
                 }
-                sm->tO[r * KM + j] = s;
-            }
+            });
             __syncthreads();
-            store_rows(x.st.K, sm->tO, r0, nr, k);
             gram_acc(sm->acc, 0, sm->tO, KM, k, sm->tO, KM, k, nr);
-            __syncthreads();
         }
-        for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-            int nr = min(TR, x.m1 - r0);
+        __syncthreads();
+        for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+            const int nr = min(tw, x.m1 - r0);
             load_rows(sm->tA, x.st.W, r0, nr, k);
+            load_mred(x, r0, nr, nullptr);
             __syncthreads();
-            for (int e = threadIdx.x; e < nr * k; e += NT) {
-                int r = e / k, j = e % k;
-                int m = r0 + r;
-                double s = 0.0;
-                for (int l = 0; l < k; ++l) s = fma(sm->tA[r * KM + l], Sm[j * KM + l], s);
-                double t = 0.0;  // (MRed P)[m][j]
-                for (int kq = 0; kq < P.q; ++kq) t = fma(P.mred[(size_t)m * P.q + kq], sm->slot[SL_P0 + 3][kq * KM + j], t);
-                sm->tO[r * KM + j] = s + dE * sig[P.lof[m]] * t;
-            }
+            for_blocks(nr, k, 0, [&](int r, int j, int o) {
+                double a[2] = {0.0, 0.0}, t[2] = {0.0, 0.0};
+                mma_dot(a, k, sm->tA + r * KM, 1, Sm + j * KM, 1);
+                mma_dot(t, P.q, sm->tP + r * QM, 1, sm->slot[SL_P0 + 3] + j, KM);   // (MRed P)[m][j]
+                if (r < nr) {
+                    const double sl = dE * sig[P.lof[r0 + r]];
+                    put_pair(sm->tO + r * KM, x.st.L + (size_t)(r0 + r) * KM, k, o, a[0] + sl * t[0], a[1] + sl * t[1]);
+                }
+            });
             __syncthreads();
-            store_rows(x.st.L, sm->tO, r0, nr, k);
             gram_acc(sm->acc, k * k, sm->tO, KM, k, sm->tO, KM, k, nr);
-            __syncthreads();
         }
         if (!publish_sync(x, 2 * k * k)) return;
         if (!range_finder(x, x.st.K, x.st.L, true, true, k)) return;
         // ---------------- phase O: new bases; MUp, X^T psi, NUp, MRed^T D W
         const int offM = 0, offXp = k * k, offN = k * k + k * P.q, offB = 2 * k * k + k * P.q;
         acc_zero(x, 2 * k * k + 2 * k * P.q);
-        for (int r0 = x.c0; r0 < x.c1; r0 += TR) {
-            int nr = min(TR, x.c1 - r0);
-            x_basis_tile(x, r0, nr, x.rhoK, k, sm->tO);
-            load_rows(sm->tA, x.st.X, r0, nr, k);
-            for (int e = threadIdx.x; e < nr * P.q; e += NT)
-                sm->tP[(e / P.q) * QM + e % P.q] = ldcg(x.psi_in + (size_t)(r0 + e / P.q) * QM + e % P.q);
-            __syncthreads();
-            gram_acc(sm->acc, offM, sm->tO, KM, k, sm->tA, KM, k, nr);
-            gram_acc(sm->acc, offXp, sm->tO, KM, k, sm->tP, QM, P.q, nr);
-            __syncthreads();
-            store_rows(x.st.X, sm->tO, r0, nr, k);
+        for (int r0 = x.c0; r0 < x.c1; r0 += tr) {
+            const int nr = min(tr, x.c1 - r0);
+            load_rows(sm->tP, x.psi_in, r0, nr, P.q, QM);
+            x_basis_tile(x, r0, nr, x.rhoK, k, sm->tO, sm->tL[0]);
+            gram_acc(sm->acc, offM, sm->tO, KM, k, sm->tL[0], KM, k, nr);
+            gram_acc(sm->acc, offXp, sm->tO, KM, k, sm->tP, QM, P.q, nr, NW / 2);
             __syncthreads();
         }
-        for (int r0 = x.m0; r0 < x.m1; r0 += TR) {
-            int nr = min(TR, x.m1 - r0);
-            w_basis_tile(x, r0, nr, x.rhoL, k - x.rhoL, sm->tO);
-            load_rows(sm->tA, x.st.W, r0, nr, k);
-            for (int e = threadIdx.x; e < nr * P.q; e += NT) {
-                int r = e / P.q, kq = e % P.q;
-                int m = r0 + r;
-                sm->tP[r * QM + kq] = P.mred[(size_t)m * P.q + kq] * sig[P.lof[m]];
-            }
-            __syncthreads();
-            gram_acc(sm->acc, offN, sm->tO, KM, k, sm->tA, KM, k, nr);
-            gram_acc(sm->acc, offB, sm->tP, QM, P.q, sm->tO, KM, k, nr);
-            __syncthreads();
-            store_rows(x.st.W, sm->tO, r0, nr, k);
+        for (int r0 = x.m0; r0 < x.m1; r0 += tw) {
+            const int nr = min(tw, x.m1 - r0);
+            load_mred(x, r0, nr, sig);
+            w_basis_tile(x, r0, nr, x.rhoL, k - x.rhoL, sm->tO, x.st.W, sm->tL[0], k);
+            gram_acc(sm->acc, offN, sm->tO, KM, k, sm->tL[0], KM, k, nr);
+            gram_acc(sm->acc, offB, sm->tP, QM, P.q, sm->tO, KM, k, nr, NW / 2);
             __syncthreads();
         }
         if (!publish_sync(x, 2 * k * k + 2 * k * P.q)) return;

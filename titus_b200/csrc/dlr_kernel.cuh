@@ -14,6 +14,14 @@
 // C = A V V2_J / nu_J materialised; CholQR on C. Directions with
 // nu_j <= tol nu_0 are null; rank-deficient bases are completed with the
 // candidate canonical vectors in index order (boundary cells for X, moments for W).
+// What bounds a step is latency: its products would take 10 us of the FP64 pipes
+// (100 x 100 cells, P_21, r = 20), but it is a chain of some 30 team barriers
+// (2 us each, 55 us), reductions through L2 (35 us), six pairs of Cholesky
+// factorisations (49 us) and, between them, short passes over a CTA's rows
+// (150 us; 290 us in all, 1060 before). So a row pass is one tile of up to TR rows
+// whose loads are one 16-byte load per thread, its products and Grams are 8 x 8
+// blocks on the FP64 tensor pipe, one per warp, and 512 threads fill those
+// blocks (256 threads with one product chain per thread took 1060 us).
 #pragma once
 #include "dlr_device.cuh"
 
@@ -56,14 +64,12 @@ struct Ctx {
     double* CW;          // N x KM scratch
     int rhoK, rhoL;
     unsigned long long* prof;  // non-null only on the profiled CTA
-    int red_mode;              // 1: reductions read the team's two-stage buffer
     unsigned gen;              // team barrier generation
     int parity;                // partial buffer in use (double-buffered)
     int cur_n;                 // energy index of the current step (diagnostics)
 };
 
 constexpr int kDirectReduceMax = 16;  // teams up to this size sum partials directly
-constexpr int kBigRows = 6 * TR;      // rows per chunk when tA..tO are used as one tile
 
 __device__ __forceinline__ bool is_bnd(const DevProblem& P, int c) {
     int i = c / P.ny, j = c - (c / P.ny) * P.ny;
@@ -85,117 +91,151 @@ __device__ __forceinline__ void acc_publish(Ctx& x, int count) {
     double* dst = part_base(x, x.b);
     for (int e = threadIdx.x; e < count; e += NT) dst[e] = x.sm->acc[e];
 }
-// sum partial entries [off, off+m*n) over the team's CTAs into dst (KM stride)
-__device__ inline void reduce_into(Ctx& x, int off, int m, int n, double* dst, int ld = KM) {
-    ProfScope ps(x.prof, PF_REDUCE);
-    if (x.red_mode) {
-        for (int e = threadIdx.x; e < m * n; e += NT) dst[(e / n) * ld + e % n] = ldcg(x.st.red + off + e);
-    } else {
-        for (int e = threadIdx.x; e < m * n; e += NT) {
-            double s = 0.0;
-            for (int g = 0; g < x.G; ++g) s += ldcg(part_base(x, g) + off + e);
-            dst[(e / n) * ld + e % n] = s;
-        }
-    }
+// entries [off, off+m*n) of the team's sums (publish_sync leaves them in acc) as a
+// matrix of KM stride
+__device__ inline void reduce_into(Ctx& x, int off, int m, int n, double* dst) {
+    for (int e = threadIdx.x; e < m * n; e += NT) dst[(e / n) * KM + e % n] = x.sm->acc[off + e];
     __syncthreads();
 }
 
-// acc[off + i*kb + j] += sum_r tA[r][i] tB[r][j]
+// acc[off + i*kb + j] += sum_{r < nr} tA[r][i] tB[r][j]; `rot` as for for_blocks.
+// Two accumulators halve the chain of products, which a block waits for.
 __device__ __forceinline__ void gram_acc(double* acc, int off, const double* tA, int lda, int ka,
-                                         const double* tB, int ldb, int kb, int nr) {
-    for (int e = threadIdx.x; e < ka * kb; e += NT) {
-        int i = e / kb, j = e - (e / kb) * kb;
-        double s = 0.0;
-        for (int r = 0; r < nr; ++r) s = fma(tA[r * lda + i], tB[r * ldb + j], s);
-        acc[off + e] += s;
-    }
+                                         const double* tB, int ldb, int kb, int nr, int rot = 0) {
+    for_blocks(ka, kb, rot, [&](int i, int j, int o) {
+        const int kr = threadIdx.x & 3;
+        double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
+#pragma unroll 1
+        for (int r0 = kr; r0 < nr + kr; r0 += 16) {
+            double av[4], bv[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const bool in = r0 + 4 * s < nr;
+                av[s] = in ? tA[(r0 + 4 * s) * lda + i] : 0.0;
+                bv[s] = in ? tB[(r0 + 4 * s) * ldb + j] : 0.0;
+            }
+            w_mma(d0, av[0], bv[0]);
+            w_mma(d1, av[1], bv[1]);
+            w_mma(d0, av[2], bv[2]);
+            w_mma(d1, av[3], bv[3]);
+        }
+        if (i < ka) {
+            if (o < kb) acc[off + i * kb + o] += d0[0] + d1[0];
+            if (o + 1 < kb) acc[off + i * kb + o + 1] += d0[1] + d1[1];
+        }
+    });
 }
 
 // ------------------------------------------------------------ row helpers ---
-__device__ __forceinline__ void load_rows(double* t, const double* A, int r0, int nr, int k) {
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        int r = e / k, j = e - (e / k) * k;
-        t[r * KM + j] = ldcg(A + (size_t)(r0 + r) * KM + j);
-    }
+// Tiles hold at most TR rows; thread t owns the columns j, j + 1 of row r of
+// such a tile, so that one load of 16 bytes a thread fetches it.
+static_assert(TR % 8 == 0 && TR * KM / 2 <= NT, "a pair of columns per thread");
+struct Pair {
+    int r, j;
+    __device__ Pair() : r(threadIdx.x / (KM / 2)), j(2 * (threadIdx.x % (KM / 2))) {}
+};
+// rows of a tile such that `rows` rows take tiles of nearly the same height
+__device__ __forceinline__ int tile_rows(int rows) {
+    const int tiles = max(1, (rows + TR - 1) / TR);
+    return max(1, (rows + tiles - 1) / tiles);
 }
-__device__ __forceinline__ void store_rows(double* A, const double* t, int r0, int nr, int k) {
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        int r = e / k, j = e - (e / k) * k;
-        A[(size_t)(r0 + r) * KM + j] = t[r * KM + j];
-    }
+__device__ __forceinline__ double2 ldcg2(const double* p) { return __ldcg(reinterpret_cast<const double2*>(p)); }
+__device__ __forceinline__ void st2(double* p, double2 v) { *reinterpret_cast<double2*>(p) = v; }
+
+// rows [r0, r0+nr) of A (row length `ld` in memory and in t), columns < k
+__device__ __forceinline__ void load_rows(double* t, const double* A, int r0, int nr, int k, int ld = KM) {
+    const Pair p;
+    if (p.r < nr && p.j < k) st2(t + p.r * ld + p.j, ldcg2(A + (size_t)(r0 + p.r) * ld + p.j));
 }
-// tO[r][j] = sum_l tA[r][l] M[l][j]  (tA: nr x ka, M: ka x kb)
-__device__ __forceinline__ void tile_mm(double* tO, const double* tA, const double* M, int nr, int ka, int kb) {
-    for (int e = threadIdx.x; e < nr * kb; e += NT) {
-        int r = e / kb, j = e - (e / kb) * kb;
-        double s = 0.0;
-        for (int l = 0; l < ka; ++l) s = fma(tA[r * KM + l], M[l * KM + j], s);
-        tO[r * KM + j] = s;
-    }
+// the pair of columns o, o + 1 of one row, of a tile and of its matrix in memory
+__device__ __forceinline__ void put_pair(double* t, double* A, int k, int o, double v0, double v1) {
+    t[o] = v0;
+    t[o + 1] = v1;
+    if (o + 1 < k) st2(A + o, make_double2(v0, v1));
+    else if (o < k) A[o] = v0;
+}
+
+// tO = tA M, also stored to rows [r0, r0+nr) of D unless D is null (tA: nr x ka, M: ka x kb)
+__device__ __forceinline__ void tile_mm(double* tO, const double* tA, const double* M, int nr, int ka, int kb,
+                                        double* D = nullptr, int r0 = 0) {
+    for_blocks(nr, kb, 0, [&](int r, int j, int o) {
+        double d[2] = {0.0, 0.0};
+        mma_dot(d, ka, tA + r * KM, 1, M + j, KM);
+        if (D && r < nr) put_pair(tO + r * KM, D + (size_t)(r0 + r) * KM, kb, o, d[0], d[1]);
+        else tO[r * KM + o] = d[0], tO[r * KM + o + 1] = d[1];
+    });
 }
 
 // Matrix-free stencils (stencils.jl:26-128) applied to rows [r0, r0+nr) of A:
-// t[0] = L2x A, t[1] = L2y A, t[2] = L1x A, t[3] = L1y A; zero on boundary rows.
-__device__ inline void stencil_tile(const Ctx& x, const double* A, int r0, int nr, int k, double (*t)[TR * KM]) {
+// t[0] = L2x A, t[1] = L2y A and, unless `central`, t[2] = L1x A, t[3] = L1y A;
+// zero on boundary rows. `tA`, if given, receives the rows of A themselves.
+__device__ inline void stencil_tile(const Ctx& x, const double* A, int r0, int nr, int k, double (*t)[TR * KM],
+                                    double* tA, bool central) {
     const DevProblem& P = x.P;
     const double hx = 0.5 / P.dx, hy = 0.5 / P.dy;
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        int r = e / k, j = e - (e / k) * k;
-        int c = r0 + r;
-        double l2x = 0.0, l2y = 0.0, l1x = 0.0, l1y = 0.0;
-        if (!is_bnd(P, c)) {
-            double a0 = ldcg(A + (size_t)c * KM + j) * P.rinv[c];
-            double axm = ldcg(A + (size_t)(c - P.ny) * KM + j) * P.rinv[c - P.ny];
-            double axp = ldcg(A + (size_t)(c + P.ny) * KM + j) * P.rinv[c + P.ny];
-            double aym = ldcg(A + (size_t)(c - 1) * KM + j) * P.rinv[c - 1];
-            double ayp = ldcg(A + (size_t)(c + 1) * KM + j) * P.rinv[c + 1];
-            l2x = (axp - axm) * hx;
-            l2y = (ayp - aym) * hy;
-            l1x = a0 / P.dx - hx * axm - hx * axp;
-            l1y = a0 / P.dy - hy * aym - hy * ayp;
-        }
-        t[0][r * KM + j] = l2x;
-        t[1][r * KM + j] = l2y;
-        t[2][r * KM + j] = l1x;
-        t[3][r * KM + j] = l1y;
+    const Pair p;
+    if (p.r >= nr || p.j >= k) return;
+    const int c = r0 + p.r, e = p.r * KM + p.j;
+    const double* a = A + (size_t)c * KM + p.j;
+    double2 l2x = {0.0, 0.0}, l2y = l2x, l1x = l2x, l1y = l2x;
+    const bool in = !is_bnd(P, c);
+    const int sx = in ? P.ny : 0, sy = in ? 1 : 0;
+    const double2 v0 = ldcg2(a), vxm = ldcg2(a - (ptrdiff_t)sx * KM), vxp = ldcg2(a + (ptrdiff_t)sx * KM),
+                  vym = ldcg2(a - sy * KM), vyp = ldcg2(a + sy * KM);
+    const double r_0 = P.rinv[c], rxm = P.rinv[c - sx], rxp = P.rinv[c + sx], rym = P.rinv[c - sy],
+                 ryp = P.rinv[c + sy];
+    if (in) {
+        const auto one = [&](double a0, double xm, double xp, double ym, double yp, double& x2, double& y2,
+                             double& x1, double& y1) {
+            const double b0 = a0 * r_0, axm = xm * rxm, axp = xp * rxp, aym = ym * rym, ayp = yp * ryp;
+            x2 = (axp - axm) * hx;
+            y2 = (ayp - aym) * hy;
+            x1 = b0 / P.dx - hx * axm - hx * axp;
+            y1 = b0 / P.dy - hy * aym - hy * ayp;
+        };
+        one(v0.x, vxm.x, vxp.x, vym.x, vyp.x, l2x.x, l2y.x, l1x.x, l1y.x);
+        one(v0.y, vxm.y, vxp.y, vym.y, vyp.y, l2x.y, l2y.y, l1x.y, l1y.y);
     }
-}
-
-// Central stencils only (the RK4 integrator's streaming): t[0] = L2x A,
-// t[1] = L2y A on rows [r0, r0+nr); zero on boundary rows.
-__device__ inline void stencil2_tile(const Ctx& x, const double* A, int r0, int nr, int k, double (*t)[TR * KM]) {
-    const DevProblem& P = x.P;
-    const double hx = 0.5 / P.dx, hy = 0.5 / P.dy;
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        int r = e / k, j = e - (e / k) * k;
-        int c = r0 + r;
-        double l2x = 0.0, l2y = 0.0;
-        if (!is_bnd(P, c)) {
-            double axm = ldcg(A + (size_t)(c - P.ny) * KM + j) * P.rinv[c - P.ny];
-            double axp = ldcg(A + (size_t)(c + P.ny) * KM + j) * P.rinv[c + P.ny];
-            double aym = ldcg(A + (size_t)(c - 1) * KM + j) * P.rinv[c - 1];
-            double ayp = ldcg(A + (size_t)(c + 1) * KM + j) * P.rinv[c + 1];
-            l2x = (axp - axm) * hx;
-            l2y = (ayp - aym) * hy;
-        }
-        t[0][r * KM + j] = l2x;
-        t[1][r * KM + j] = l2y;
+    if (tA) st2(tA + e, v0);
+    st2(t[0] + e, l2x);
+    st2(t[1] + e, l2y);
+    if (!central) {
+        st2(t[2] + e, l1x);
+        st2(t[3] + e, l1y);
     }
 }
 
 // Sparse P_N operators applied to rows [r0, r0+nr) of B (N x KM): t[d] = A_d B
-// for the first `nops` operators (Ax, Az, |Ax|, |Az|).
+// for the first `nops` operators (Ax, Az, |Ax|, |Az|). Four entries of a row are
+// in flight at a time; those past its end repeat the first one with weight zero.
 __device__ inline void spmm_tile(const Ctx& x, const double* B, int r0, int nr, int k, double (*t)[TR * KM],
                                  int nops = NOPS) {
-    for (int e = threadIdx.x; e < nops * nr * k; e += NT) {
-        int d = e / (nr * k);
-        int rem = e - d * nr * k;
-        int r = rem / k, j = rem - (rem / k) * k;
+    const int kp = (k + 1) >> 1;
+    for (int e = threadIdx.x; e < nops * nr * kp; e += NT) {
+        const int d = e / (nr * kp), rem = e - d * nr * kp;
+        const int r = rem / kp, j = 2 * (rem - r * kp);
         const Csr& A = x.P.op[d];
-        int m = r0 + r;
-        double s = 0.0;
-        for (int p = A.rowptr[m]; p < A.rowptr[m + 1]; ++p) s = fma(A.val[p], ldcg(B + (size_t)A.col[p] * KM + j), s);
-        t[d][r * KM + j] = s;
+        const int p0 = A.rowptr[r0 + r], p1 = A.rowptr[r0 + r + 1];
+        double2 s = {0.0, 0.0};
+#pragma unroll 1
+        for (int p = p0; p < p1; p += 4) {
+            int col[4];
+            double val[4];
+            double2 b[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                col[u] = A.col[p + u < p1 ? p + u : p];
+                val[u] = p + u < p1 ? A.val[p + u] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) b[u] = ldcg2(B + (size_t)col[u] * KM + j);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                s.x = fma(val[u], b[u].x, s.x);
+                s.y = fma(val[u], b[u].y, s.y);
+            }
+        }
+        st2(t[d] + r * KM + j, s);
     }
 }
 
@@ -293,21 +333,17 @@ static __device__ __noinline__ void w_complete(Ctx& x, int rho, int need) {
     }
 }
 
-// Materialise rows [r0, r0+nr) of the new W-side basis into tile t:
-// columns :rho = C Ri, columns rho+a = completion vector a.
-__device__ inline void w_basis_tile(Ctx& x, int r0, int nr, int rho, int need, double* t) {
+// Materialise rows [r0, r0+nr) of the new W-side basis into tile t and of `old`,
+// if given, into tile tB: columns :rho = C Ri, columns rho+a = completion vector a.
+__device__ inline void w_basis_tile(Ctx& x, int r0, int nr, int rho, int need, double* t, const double* old = nullptr,
+                                    double* tB = nullptr, int k = 0) {
     SmemLayout* sm = x.sm;
-    const double* Ri = sm->slot[SL_RIL];
     load_rows(sm->tA, x.CW, r0, nr, rho);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nr * rho; e += NT) {
-        int r = e / rho, j = e - (e / rho) * rho;
-        double s = 0.0;
-        for (int l = 0; l <= j; ++l) s = fma(sm->tA[r * KM + l], Ri[l * KM + j], s);
-        t[r * KM + j] = s;
-    }
+    if (old) load_rows(tB, old, r0, nr, k);
     __syncthreads();
     if (need > 0) {
+        tile_mm(t, sm->tA, sm->slot[SL_RIL], nr, rho, rho);
+        __syncthreads();
         const double* wc = sm->slot[SL_WC];
         for (int r = threadIdx.x; r < nr; r += NT) {
             int m = r0 + r;
@@ -320,28 +356,34 @@ __device__ inline void w_basis_tile(Ctx& x, int r0, int nr, int rho, int need, d
             }
         }
         __syncthreads();
+        const Pair p;
+        if (p.r < nr && p.j < rho + need)
+            put_pair(t + p.r * KM, x.st.W + (size_t)(r0 + p.r) * KM, rho + need, p.j, t[p.r * KM + p.j],
+                     t[p.r * KM + p.j + 1]);
+    } else {
+        tile_mm(t, sm->tA, sm->slot[SL_RIL], nr, rho, rho, x.st.W, r0);
     }
+    __syncthreads();
 }
 
-// Materialise rows of the new X-side basis: C Ri, then completion cells.
-__device__ inline void x_basis_tile(Ctx& x, int r0, int nr, int rho, int k, double* t) {
+// Materialise rows of the new X-side basis into tile t and X, and the old ones
+// into tile tB: C Ri, then completion cells.
+__device__ inline void x_basis_tile(Ctx& x, int r0, int nr, int rho, int k, double* t, double* tB) {
     SmemLayout* sm = x.sm;
-    const double* Ri = sm->slot[SL_RIK];
     load_rows(sm->tA, x.CX, r0, nr, rho);
+    load_rows(tB, x.st.X, r0, nr, k);
     __syncthreads();
-    for (int e = threadIdx.x; e < nr * k; e += NT) {
-        int r = e / k, j = e - (e / k) * k;
-        double s;
-        if (j < rho) {
-            s = 0.0;
-            for (int l = 0; l <= j; ++l) s = fma(sm->tA[r * KM + l], Ri[l * KM + j], s);
-        } else {
-            // completion failures are reported through the status flag; keep reads in bounds
-            const int ci = j - rho;
-            s = (ci < x.P.nxcomp && r0 + r == x.P.xcomp[ci]) ? 1.0 : 0.0;
+    for_blocks(nr, k, 0, [&](int r, int j, int o) {
+        double d[2] = {0.0, 0.0};
+        mma_dot(d, rho, sm->tA + r * KM, 1, sm->slot[SL_RIK] + j, KM);
+        if (r >= nr) return;
+        // completion failures are reported through the status flag; keep reads in bounds
+        for (int h = 0; h < 2; ++h) {
+            const int ci = o + h - rho;
+            if (ci >= 0) d[h] = (ci < x.P.nxcomp && r0 + r == x.P.xcomp[ci]) ? 1.0 : 0.0;
         }
-        t[r * KM + j] = s;
-    }
+        put_pair(t + r * KM, x.st.X + (size_t)(r0 + r) * KM, k, o, d[0], d[1]);
+    });
     __syncthreads();
 }
 

@@ -333,15 +333,6 @@ __device__ __forceinline__ void wstore(double* A, int lda, int c0, const double*
     for (RowWalk x(k); x.r < nr; x.next()) A[(size_t)(r0 + x.r) * lda + c0 + x.j] = t[x.r * ldt + tc + x.j];
 }
 
-// D += A B on an 8 x 8 tile, four columns of A at a time (FP64 tensor pipe): a
-// lane holds A[lane / 4][lane % 4], B[lane % 4][lane / 4] and
-// D[lane / 4][2 (lane % 4) + {0, 1}].
-__device__ __forceinline__ void w_mma(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
-
 // Row products of a shared-memory tile: for rows r < nr and columns j < w,
 //   epi(r, j, sum_{l < kd} A[r * lda + l] * mget(l, j)).
 // A warp takes 16 rows x 8 columns and walks l in steps of four on the FP64
