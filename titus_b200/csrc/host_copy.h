@@ -1,0 +1,146 @@
+// Device-to-host copies of large results into pageable memory.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstddef>
+#include <cstring>
+#include <mutex>
+#include <thread>
+
+namespace titus_host {
+
+// cudaMemcpy2D to pageable memory goes through one thread, which takes every page
+// fault of a fresh result array and copies row by row (40 000 rows of 19 values
+// into rows of 80: 20 ms; 40 000 x 900 contiguous: 78 ms, 18 when the pages are
+// there). Here up to kThreads threads take a span of the rows each and copy it by
+// chunks through two pinned buffers of their own, one chunk in flight while the
+// other is scattered. Spans, not chunks dealt in turn: threads that write to one
+// huge page fault it together, and 6 MB of fresh contiguous rows then took 5 to 11
+// ms instead of 0.4. The buffers (4 MiB in all), streams
+// and the events are made by the first large copy of a handle and freed with it.
+// From kLarge bytes of strided destination on (8 MB: 6.1 -> 1.2 ms into fresh pages,
+// 4.2 -> 0.3 into touched ones; the first copy of a handle, which makes the buffers,
+// 5 ms) and kLargeFlat of contiguous (32 MB: 14 -> 2.6 ms fresh, 2.0 -> 1.7 touched;
+// at 8 MB touched 0.5 either way, and pages of 2 MB are cheap to fault in one go).
+// Device work that writes the source must have completed.
+class HostCopy {
+public:
+    static constexpr int kThreads = 8;
+    static constexpr size_t kChunk = 256u << 10, kSpan = 2u << 20, kLarge = 4u << 20, kLargeFlat = 16u << 20;
+
+    // the row-wise copy of cudaMemcpy2D(..., cudaMemcpyDeviceToHost), pitches in bytes
+    cudaError_t copy2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t height) {
+        const size_t bytes = height * dpitch;
+        if (bytes < (dpitch == width ? kLargeFlat : kLarge) || width == 0 || width > kChunk)
+            return cudaMemcpy2D(dst, dpitch, src, spitch, width, height, cudaMemcpyDeviceToHost);
+        std::lock_guard<std::mutex> hold(lock_);
+        const int nt = lanes((int)std::min<size_t>(kThreads, bytes / kSpan));
+        if (nt < 2) return cudaMemcpy2D(dst, dpitch, src, spitch, width, height, cudaMemcpyDeviceToHost);
+        int device = 0;
+        cudaError_t rc = cudaGetDevice(&device);
+        if (rc != cudaSuccess) return rc;
+        const size_t rows = kChunk / width, span = (height + nt - 1) / nt;
+        std::atomic<int> part{0};
+        std::atomic<int> err{(int)cudaSuccess};
+        const auto work = [&](Lane* L) {
+            cudaError_t e = cudaSetDevice(device);
+            for (int p; (p = part.fetch_add(1)) < nt && e == cudaSuccess;) {
+                const size_t end = std::min(height, (p + 1) * span);
+                size_t next = std::min(height, p * span), at[2] = {end, end};
+                const auto fetch = [&](int b) {
+                    at[b] = next;
+                    if (next == end || e != cudaSuccess) return;
+                    const size_t n = std::min(rows, end - next);
+                    const char* s = static_cast<const char*>(src) + next * spitch;
+                    next += n;
+                    e = spitch == width ? cudaMemcpyAsync(L->buf[b], s, n * width, cudaMemcpyDeviceToHost, L->stream)
+                                        : cudaMemcpy2DAsync(L->buf[b], width, s, spitch, width, n, cudaMemcpyDeviceToHost,
+                                                            L->stream);
+                    if (e == cudaSuccess) e = cudaEventRecord(L->done[b], L->stream);
+                };
+                fetch(0);
+                for (int b = 0; at[b] < end && e == cudaSuccess; b ^= 1) {
+                    fetch(b ^ 1);
+                    if (e == cudaSuccess) e = cudaEventSynchronize(L->done[b]);
+                    if (e != cudaSuccess) break;
+                    const size_t n = std::min(rows, end - at[b]);
+                    char* d = static_cast<char*>(dst) + at[b] * dpitch;
+                    if (dpitch == width) {
+                        std::memcpy(d, L->buf[b], n * width);
+                    } else {
+                        for (size_t r = 0; r < n; ++r) std::memcpy(d + r * dpitch, L->buf[b] + r * width, width);
+                    }
+                    at[b] = end;
+                }
+            }
+            if (e != cudaSuccess) {
+                cudaStreamSynchronize(L->stream);   // nothing in flight into the buffers
+                err.store((int)e);
+            }
+        };
+        std::thread th[kThreads - 1];
+        int started = 0;
+        try {
+            for (; started < nt - 1; ++started) th[started] = std::thread(work, &lane_[started + 1]);
+        } catch (...) {   // no more threads: those that run, and this one, take all rows
+        }
+        work(&lane_[0]);
+        for (int t = 0; t < started; ++t) th[t].join();
+        return (cudaError_t)err.load();
+    }
+
+    void release() {
+        for (Lane& L : lane_)
+            for (int b = 0; b < 2; ++b)
+                if (L.done[b]) cudaEventDestroy(L.done[b]);
+        for (cudaStream_t& st : stream_) {
+            if (st) cudaStreamDestroy(st);
+            st = nullptr;
+        }
+        if (pinned_) cudaFreeHost(pinned_);
+        for (Lane& L : lane_) L = Lane{};
+        pinned_ = nullptr;
+        ready_ = false;
+    }
+
+private:
+    struct Lane {
+        cudaEvent_t done[2] = {nullptr, nullptr};
+        char* buf[2] = {nullptr, nullptr};
+        cudaStream_t stream = nullptr;
+    };
+    Lane lane_[kThreads];
+    cudaStream_t stream_[2] = {nullptr, nullptr};   // of the even and the odd lanes: two keep the copy engines busy
+    char* pinned_ = nullptr;
+    bool ready_ = false;
+    std::mutex lock_;
+
+    // the lanes that can be used: none (the plain copy serves) when something runs out
+    int lanes(int want) {
+        want = (int)std::min<unsigned>(want, std::max(1u, std::thread::hardware_concurrency()));
+        if (want < 2) return 0;
+        if (!ready_ && !make()) {
+            cudaGetLastError();
+            release();
+            return 0;
+        }
+        ready_ = true;
+        return want;
+    }
+    bool make() {
+        if (cudaHostAlloc((void**)&pinned_, kThreads * 2 * kChunk, cudaHostAllocPortable) != cudaSuccess) return false;
+        for (cudaStream_t& st : stream_)
+            if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return false;
+        for (int t = 0; t < 2 * kThreads; ++t) {
+            Lane& L = lane_[t / 2];
+            L.buf[t % 2] = pinned_ + t * kChunk;
+            L.stream = stream_[(t / 2) % 2];
+            if (cudaEventCreateWithFlags(&L.done[t % 2], cudaEventDisableTiming) != cudaSuccess) return false;
+        }
+        return true;
+    }
+};
+
+}  // namespace titus_host

@@ -259,8 +259,7 @@ int titus_host::TITUS_WIDE_HOST(wide_fetch)(titus_solver* s, titus_result_t* res
     const int cap = res->r_cap;
     if ((res->X || res->S || res->W) && cap < k) return fail(TITUS_ERR_ARG, "r_cap %d < rank %d", cap, k);
     if (res->X)
-        CK(cudaMemcpy2D(res->X, cap * sizeof(double), w.X, KA * sizeof(double), k * sizeof(double), s->n,
-                        cudaMemcpyDeviceToHost));
+        CK(s->host_copy.copy2d(res->X, cap * sizeof(double), w.X, KA * sizeof(double), k * sizeof(double), s->n));
     if (res->W)
         CK(cudaMemcpy2D(res->W, cap * sizeof(double), w.W, KA * sizeof(double), k * sizeof(double), s->N,
                         cudaMemcpyDeviceToHost));
@@ -269,8 +268,8 @@ int titus_host::TITUS_WIDE_HOST(wide_fetch)(titus_solver* s, titus_result_t* res
                         cudaMemcpyDeviceToHost));
     if (res->psi) {
         double* src = info[2] ? w.psi1 : w.psi0;
-        CK(cudaMemcpy2D(res->psi, s->q * sizeof(double), src, QW * sizeof(double), s->q * sizeof(double), s->n,
-                        cudaMemcpyDeviceToHost));
+        CK(s->host_copy.copy2d(res->psi, s->q * sizeof(double), src, QW * sizeof(double), s->q * sizeof(double),
+                               s->n));
     }
     const int nh = std::min(s->nE, w.hist_cap);
     if (res->rank_history) CK(cudaMemcpy(res->rank_history, w.rank_hist, nh * sizeof(int), cudaMemcpyDeviceToHost));

@@ -45,6 +45,7 @@ titus_solver::~titus_solver() {
     titus_host::pn_free(this);
     titus_host::pn3_free(this);
     titus_host::wide_free(this);
+    host_copy.release();
     for (void* p : allocs) cudaFree(p);
 }
 
@@ -474,8 +475,8 @@ extern "C" int titus_fetch(titus_solver_t* s, titus_result_t* res) {
     const int rc_cap = res->r_cap;
     if ((res->X || res->S || res->W) && rc_cap < k) return fail(TITUS_ERR_ARG, "r_cap %d < rank %d", rc_cap, k);
     if (res->X)
-        CK(cudaMemcpy2D(res->X, rc_cap * sizeof(double), s->st.X, KM * sizeof(double), k * sizeof(double), s->n,
-                        cudaMemcpyDeviceToHost));
+        CK(s->host_copy.copy2d(res->X, rc_cap * sizeof(double), s->st.X, KM * sizeof(double), k * sizeof(double),
+                               s->n));
     if (res->W)
         CK(cudaMemcpy2D(res->W, rc_cap * sizeof(double), s->st.W, KM * sizeof(double), k * sizeof(double), s->N,
                         cudaMemcpyDeviceToHost));
@@ -484,8 +485,8 @@ extern "C" int titus_fetch(titus_solver_t* s, titus_result_t* res) {
                         cudaMemcpyDeviceToHost));
     if (res->psi) {
         double* src = info[2] ? s->st.psi1 : s->st.psi0;
-        CK(cudaMemcpy2D(res->psi, s->q * sizeof(double), src, QM * sizeof(double), s->q * sizeof(double), s->n,
-                        cudaMemcpyDeviceToHost));
+        CK(s->host_copy.copy2d(res->psi, s->q * sizeof(double), src, QM * sizeof(double), s->q * sizeof(double),
+                               s->n));
     }
     if (res->rank_history) CK(cudaMemcpy(res->rank_history, s->st.rank_hist, s->nE * sizeof(int), cudaMemcpyDeviceToHost));
     if (res->eta_history) memset(res->eta_history, 0, s->nE * sizeof(double));

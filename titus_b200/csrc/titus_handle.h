@@ -6,6 +6,7 @@
 
 #include "../../include/titus.h"
 #include "dlr_device.cuh"
+#include "host_copy.h"
 #include "wide_state.h"
 
 struct titus_solver;
@@ -106,6 +107,7 @@ struct titus_solver {
     // test hook (titus_debug_barrier_fault), consumed by the next launch
     long long dbg_spin_limit = 0;
     int dbg_fault_barrier = 0;
+    titus_host::HostCopy host_copy;   // large results to the host
     void take_debug_hooks(titus::DevProblem& P) {
         P.spin_limit = dbg_spin_limit;
         P.fault_barrier = dbg_fault_barrier;

@@ -174,7 +174,9 @@ int titus_host::pn3_fetch(titus_solver* s, double* u_out, double* dose_out, doub
         titus_pn::pt_unpack_kernel<<<s->num_sms * 8, P3_NT>>>(s->n, s->N, st->layout.ldu, st->col_of,
                                                               st->u[st->cur_u], tmp);
         CK(cudaGetLastError());
-        CK(cudaMemcpy(u_out, tmp, (size_t)s->n * s->N * sizeof(double), cudaMemcpyDeviceToHost));
+        CK(cudaDeviceSynchronize());
+        const size_t row = (size_t)s->N * sizeof(double);
+        CK(s->host_copy.copy2d(u_out, row, tmp, row, row, s->n));
     }
     if (dose_out) CK(cudaMemcpy(dose_out, st->dose, (size_t)s->n * sizeof(double), cudaMemcpyDeviceToHost));
     if (psi_out)

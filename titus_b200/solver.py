@@ -493,7 +493,8 @@ def SolveFirstCollisionSource(solver: SolverCSD, max_steps: int = 0):
     _lib.check(lib.titus_pn_full_solve(h, C.byref(opt), _lib.as_dp(u), _lib.as_dp(dose), _lib.as_dp(psi)),
                "titus_pn_full_solve")
     solver.dose = dose
-    return 0.5 * math.sqrt(solver.gamma[0]) * u, dose, psi.reshape(solver.psi_shape)
+    u *= 0.5 * math.sqrt(solver.gamma[0])
+    return u, dose, psi.reshape(solver.psi_shape)
 
 
 def DoseAdjoint(solver: SolverCSD, weight=None, target=None, dj_ddose=None, checkpoint_every: int = 0,
