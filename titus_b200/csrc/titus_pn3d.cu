@@ -32,7 +32,9 @@ constexpr int P3_NOP = 6;
 // Largest moment count taken (P64).
 constexpr int P3_MAX_MOMENTS = 4266;
 
-// 4 x 2 x 8 cells, 48 operator tiles a stage.
+// 4 x 2 x 8 cells, 56 operator tiles a stage, two CTAs a SM: as many tiles as fit beside
+// the stencil coefficients and the larger halo in shared memory (64^3, P13: 1667 us a
+// step with 48 tiles, 1584 with 64 and the coefficients in registers, 1538 so).
 using Shape3D = titus_pn::PtShape<3, 1, 4, 2, 56, 2>;
 
 }  // namespace

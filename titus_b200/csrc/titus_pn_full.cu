@@ -30,7 +30,9 @@ constexpr int PN_NT = 256;    // threads per CTA of the cell-wise kernels
 // Largest moment counts taken (P59 forward, P39 adjoint).
 constexpr int PN_MAX_MOMENTS = 3632, ADJ_MAX_MOMENTS = 1600;
 
-// 8 x 8 cells, 80 operator tiles a stage.
+// 8 x 8 cells, 96 operator tiles a stage, two CTAs a SM: as many tiles as fit beside
+// the stencil coefficients in shared memory (200 x 200, P29: 1255 us a step with 80
+// tiles, 1132 with 112 and the coefficients in registers, 1086 so).
 using Shape2D = titus_pn::PtShape<2, 1, 1, 8, 96, 2>;
 
 }  // namespace
