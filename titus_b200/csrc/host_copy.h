@@ -20,20 +20,20 @@ namespace titus_host {
 // huge page fault it together, and 6 MB of fresh contiguous rows then took 5 to 11
 // ms instead of 0.4. The buffers (4 MiB in all), streams
 // and the events are made by the first large copy of a handle and freed with it.
-// From kLarge bytes of strided destination on (8 MB: 6.1 -> 1.2 ms into fresh pages,
-// 4.2 -> 0.3 into touched ones; the first copy of a handle, which makes the buffers,
-// 5 ms) and kLargeFlat of contiguous (32 MB: 14 -> 2.6 ms fresh, 2.0 -> 1.7 touched;
-// at 8 MB touched 0.5 either way, and pages of 2 MB are cheap to fault in one go).
+// From kLarge bytes of destination on (32 MB into fresh pages: strided 26 -> 1.9 ms,
+// contiguous 14 -> 2.6; into touched ones 16.5 -> 0.7 and 2.0 -> 1.7). 8 MB of strided
+// rows would gain as well when repeated (6.1 -> 1.2 ms), but a handle's first copy,
+// which makes the buffers, costs 5 ms and more, and counts as much.
 // Device work that writes the source must have completed.
 class HostCopy {
 public:
     static constexpr int kThreads = 8;
-    static constexpr size_t kChunk = 256u << 10, kSpan = 2u << 20, kLarge = 4u << 20, kLargeFlat = 16u << 20;
+    static constexpr size_t kChunk = 256u << 10, kSpan = 2u << 20, kLarge = 16u << 20;
 
     // the row-wise copy of cudaMemcpy2D(..., cudaMemcpyDeviceToHost), pitches in bytes
     cudaError_t copy2d(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t height) {
         const size_t bytes = height * dpitch;
-        if (bytes < (dpitch == width ? kLargeFlat : kLarge) || width == 0 || width > kChunk)
+        if (bytes < kLarge || width == 0 || width > kChunk)
             return cudaMemcpy2D(dst, dpitch, src, spitch, width, height, cudaMemcpyDeviceToHost);
         std::lock_guard<std::mutex> hold(lock_);
         const int nt = lanes((int)std::min<size_t>(kThreads, bytes / kSpan));
