@@ -214,7 +214,7 @@ static int create_impl(const titus_problem_t* pb, titus_solver* s, int nz = 0) {
     }
     // team state (one team); partial buffer sized for the largest team
     // Default team: one tile of rows per CTA. Fewer CTAs walk several tiles one after
-    // the other (100 x 100, P21, r = 20: 340 us a step with 148 CTAs, 630 with 32),
+    // the other (100 x 100, P21, r = 20: 357 us a step with 148 CTAs, 507 with 32),
     // more only lengthen the reductions (24 x 24, P5, r = 8: 173 us with 16, 188
     // with 32, where sums over more than 16 CTAs take a second stage, 198 with 148).
     s->team_ctas = std::min(s->num_sms, std::max(kDirectReduceMax, (s->n + TR - 1) / TR));
