@@ -516,15 +516,9 @@ def run_gpu_pn_full(args, w, rank, world, local_rank, dist):
     e2e_value, _ = replica_throughput(1, time.perf_counter() - t0, world, device="cuda")
     steps = solver.nE - 1
     nN = solver.n * solver.N
-    if three_d:
-        # per step, the fused stencil + moment kernel reads u and writes u' (2 nN); psi is
-        # written by the sweep and read by the sweep and the stream kernel (3 n q); the
-        # dose is read and written and 1/rho read once (3 n)
-        alg = steps * 8 * (2 * nN + 3 * solver.n * solver.q + 3 * solver.n)
-    else:
-        # per step: moments read u, write W (5 nN); stream reads u, W (4 nN), writes u' (6 nN);
-        # psi read + write (2 n q), dose read + write (2 n)
-        alg = steps * 8 * (11 * nN + 2 * solver.n * solver.q + 2 * solver.n)
+    # per step the one kernel reads u and psi and writes u' and psi' (2 nN + 2 n q); the
+    # dose is read and written and 1/rho read once (3 n)
+    alg = steps * 8 * (2 * nN + 2 * solver.n * solver.q + 3 * solver.n)
     peak, peak_kind = read_peaks()
     achieved = alg / (t_max / args.steps) / 1e9
     info = dict(value=value, ms_per_step=t_max / args.steps * 1e3, e2e_value=e2e_value, h2d=h2d, d2h=d2h,
@@ -823,7 +817,8 @@ def run_gpu(args, w, rank, world, local_rank):
                                  "peak_kind": info["peak_kind"], "algorithmic_bytes_per_launch": info["alg"],
                                  "note": "all kernels of every energy step (one graph launch)"},
                     "clocks": info["clocks"],
-                    "gpu_launches": (2 if args.method == "pn3d" else 3) * info["steps_per_solve"] * args.steps,
+                    # per solve: one kernel an energy step and the boundary ordinates of the last
+                    "gpu_launches": (info["steps_per_solve"] + 1) * args.steps,
                     "dose_max": info["dose_max"], "cpu_baseline": None}
             if world == 1 and not args.no_cpu_baseline:
                 cores = host_threads()
