@@ -139,3 +139,27 @@ def test_step_3d(nx, ny, nz, npn):
     assert rel(u, 0.5 * np.sqrt(2.0) * ref[0]) <= TOL
     assert rel(dose, ref[1]) <= TOL
     assert rel(psi, ref[2]) <= TOL
+
+
+def test_adjoint_without_entries_in_a_column_group():
+    """Operators that hold nothing outside the first 60 of 196 moments: the second column group of the tiled
+    kernel (13 of its 25 output tiles) has no chunk in the adjoint, and its columns decay by the collision alone."""
+    sv = solver2d(34, 34, 13)
+    rng = np.random.default_rng(8)
+    ops = []
+    for _ in range(4):
+        A = np.zeros((sv.N, sv.N))
+        A[:60, :60] = rng.standard_normal((60, 60)) / (2 * np.sqrt(60))
+        ops.append(ph.to_csr(A))
+    sv.ops = ops
+    nnz = sum(len(v) for _, _, v in ops)
+    assert 32 * 32 * nnz > 10**7               # beyond the small kernel's range
+    w, t = rng.uniform(0.5, 1.5, sv.n), rng.uniform(0.0, 1.0, sv.n)
+    J, dose, grho, gprof = DoseAdjoint(sv, w, t, checkpoint_every=2, max_steps=5)
+    density = torch.from_numpy(sv.density).cuda().requires_grad_(True)
+    profile = torch.from_numpy(sv.bc_space).cuda().requires_grad_(True)
+    _, d, _ = sweep(sv, 5, density, profile)
+    Jr = (torch.from_numpy(w).cuda() * (d - torch.from_numpy(t).cuda()) ** 2).sum()
+    Jr.backward()
+    assert abs(J - Jr.item()) <= TOL * abs(Jr.item())
+    assert rel(dose, d) <= TOL and rel(grho, density.grad) <= TOL and rel(gprof, profile.grad) <= TOL

@@ -459,6 +459,9 @@ __global__ void __launch_bounds__(S::NTHR, S::CTAS)
         }
     }
 
+    // the column constants come from other threads: the chunk loop's barriers order them, unless no operator
+    // has an entry in these columns (an adjoint group without chunks)
+    if (nchunks == 0) __syncthreads();
     // epilogue: lane holds columns 2 kl + {0, 1} of every tile for its cells
     double dcell[MT];
 #pragma unroll
