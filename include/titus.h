@@ -99,7 +99,10 @@ typedef struct titus_problem {
 typedef enum titus_precision { TITUS_PRECISION_FP64 = 0, TITUS_PRECISION_MIXED = 1 } titus_precision_t;
 
 typedef struct titus_options {
-    int32_t team_ctas;     /* CTAs cooperating on one solve (0 = library default) */
+    int32_t team_ctas;     /* CTAs cooperating on one solve, one per SM (0 = library default: by the
+                              problem's size up to the whole GPU on the default stream, and at most 32
+                              (fixed rank, RK4) or 64 (rank-adaptive) on a stream of the caller's own,
+                              so that solves of several handles run side by side) */
     int32_t max_steps;     /* stop after this many loop iterations (0 = full sweep) */
     double rank_tol;       /* relative singular-value cut for numerical rank (0 = 1e-12) */
     int32_t profile;       /* 1 = record per-phase device timers (read with titus_profile) */

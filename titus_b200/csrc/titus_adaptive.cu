@@ -121,12 +121,14 @@ int init_state(titus_solver* s, int r0, int method, cudaStream_t stream) {
 
 int launch(titus_solver* s, int method, const titus_options_t* opt, int n_begin, int n_end, int max_iters,
            cudaStream_t stream) {
-    // Default team: one CTA per hundred cells, at least 64. Below that a CTA's rows
+    // Default team (of a solve that has the chip to itself; 64 on a caller's own stream, see
+    // default_team): one CTA per hundred cells, at least 64. Below that a CTA's rows
     // are one tile and more CTAs only lengthen the reductions and barriers (48 x 48,
     // P7, rank 20: 539 us a step with 64 CTAs, 571 with 148); above, the rows are
     // the step (200 x 200, P29, rank 80: 2900 us with 64, 2380 with 148; 100 x 100:
     // 987 with 100, 1009 with 64).
-    int G = (opt && opt->team_ctas > 0) ? opt->team_ctas : std::max(64, (s->n + 99) / 100);
+    int G = (opt && opt->team_ctas > 0) ? opt->team_ctas
+                                        : titus_host::default_team(std::max(64, (s->n + 99) / 100), 64, stream);
     G = std::max(1, std::min(G, s->num_sms));
     int per_sm = 0;
     const KernelFn kfun = kernel_for<kThreeD>(method);

@@ -213,7 +213,7 @@ static int create_impl(const titus_problem_t* pb, titus_solver* s, int nz = 0) {
         P.op[d].val = v;
     }
     // team state (one team); partial buffer sized for the largest team
-    // Default team: one tile of rows per CTA. Fewer CTAs walk several tiles one after
+    // Default team (of a solve that has the chip to itself, see default_team): one tile of rows per CTA. Fewer CTAs walk several tiles one after
     // the other (100 x 100, P21, r = 20: 357 us a step with 148 CTAs, 507 with 32),
     // more only lengthen the reductions (24 x 24, P5, r = 8: 173 us with 16, 188
     // with 32, where sums over more than 16 CTAs take a second stage, 198 with 148).
@@ -371,7 +371,7 @@ static int launch(titus_solver* s, int method, const titus_options_t* opt, int n
         if (rc) return rc;
     }
     void* kfn = ho ? (void*)dlr_kernel<TITUS_DLR_HIGH_ORDER> : (void*)dlr_kernel<TITUS_DLR_FIXED>;
-    int G = (opt && opt->team_ctas > 0) ? opt->team_ctas : s->team_ctas;
+    int G = (opt && opt->team_ctas > 0) ? opt->team_ctas : titus_host::default_team(s->team_ctas, 32, stream);
     G = std::min(G, s->num_sms);
     G = std::max(G, 1);
     int per_sm = 0;
