@@ -83,16 +83,19 @@ extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(
 }
 
 // h rows of w doubles, from rows of sp into rows of dp
-static int check(const char* what, size_t w, size_t sp, size_t dp, size_t h, bool staged) {
-    std::vector<double> src(sp * h), dst(dp * h, 7.5);
+static int check(const char* what, size_t w, size_t sp, size_t dp, size_t h, bool staged, bool fresh = false) {
+    std::vector<double> src(sp * h);
+    auto* dst = (double*)mmap(nullptr, dp * h * 8, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (!fresh) std::fill_n(dst, dp * h, 7.5);
     for (size_t i = 0; i < src.size(); ++i) src[i] = (double)i;
     titus_host::HostCopy copy;
     fake.plain = fake.staged = 0;
-    const int rc = copy.copy2d(dst.data(), dp * 8, src.data(), sp * 8, w * 8, h);
+    const int rc = copy.copy2d(dst, dp * 8, src.data(), sp * 8, w * 8, h);
     copy.release();
     bool same = rc == 0;
     for (size_t r = 0; r < h && same; ++r)
         for (size_t j = 0; j < dp && same; ++j) same = dst[r * dp + j] == (j < w ? src[r * sp + j] : 7.5);
+    munmap(dst, dp * h * 8);
     const bool way = staged ? fake.plain == 0 && fake.staged > 0 : fake.plain == 1 && fake.staged == 0;
     if (!same || !way) printf("%s: rc %d, bytes %s, %d plain, %d staged\n", what, rc, same ? "equal" : "differ",
                               (int)fake.plain, (int)fake.staged);
@@ -102,19 +105,22 @@ int main() {
     const bool lanes = std::thread::hardware_concurrency() > 1;
     int bad = check("small", 19, 80, 80, 1000, false);
     bad += check("strided", 19, 80, 80, 40001, lanes);
-    bad += check("contiguous", 900, 900, 900, 2503, lanes);
+    bad += check("contiguous, pages there", 900, 900, 900, 4503, false);
+    bad += check("contiguous, fresh pages", 900, 900, 900, 4503, lanes, true);
+    bad += check("contiguous from strided rows, fresh pages", 20, 24, 20, 220001, lanes, true);
+    bad += check("contiguous, pages there, 144 MB", 900, 900, 900, 20003, lanes);
     bad += check("wide rows", 40000, 40000, 40000, 57, false);
     fake.threads_left = 2;
     bad += check("two more threads", 19, 80, 80, 40001, lanes);
     fake.threads_left = 0;
-    bad += check("no more threads", 900, 900, 900, 2503, lanes);
+    bad += check("no more threads", 900, 900, 900, 4503, lanes, true);
     fake.threads_left = 1 << 20;
     fake.no_pool = true;
     bad += check("no buffers", 19, 80, 80, 40001, false);
     fake.no_pool = false;
     fake.pinned = true;
     bad += check("pinned, strided", 19, 80, 80, 40001, false);
-    bad += check("pinned, contiguous", 900, 900, 900, 2503, false);
+    bad += check("pinned, contiguous", 900, 900, 900, 20003, false);
     return bad;
 }
 """
