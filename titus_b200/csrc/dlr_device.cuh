@@ -15,7 +15,9 @@ namespace titus {
 constexpr int NT = 512;        // threads per CTA
 constexpr int NW = NT / 32;    // warps per CTA
 constexpr int KM = 24;         // max basis width handled by this build
-constexpr int QM = 32;         // max reduced ordinates
+constexpr int QM = 32;         // row length of the reduced ordinates in memory
+constexpr int QMAX = QM < KM ? QM : KM;   // most reduced ordinates a problem may have: the fixed-rank kernel's row
+                                          // loads and products take at most KM columns
 constexpr int TR = 40;         // rows per staged tile: one pair of columns per thread
 constexpr int NOPS = 4;        // Ax, Az, |Ax|, |Az|
 constexpr int KK = KM * KM;
@@ -228,6 +230,7 @@ __device__ __forceinline__ void for_blocks(int m, int n, int rot, F f) {
 // the chain of products is what a block waits for, and a loop over l of unknown
 // length costs more than its six steps. Columns past kd count as zero.
 __device__ __forceinline__ void mma_dot(double (&d)[2], int kd, const double* a, int sa, const double* b, int sb) {
+    static_assert(QMAX <= KM && KM % 8 == 0, "kd may be the number of ordinates; two steps of four at a time");
     const int kr = threadIdx.x & 3;
     double av[KM / 4], bv[KM / 4];
 #pragma unroll

@@ -87,7 +87,8 @@ __device__ inline void phase_bc_dose(Ctx& x, int n, bool dose2_pending, bool do_
     double* v = sm->vec;  // S W[0,:]^T
     double* w0 = sm->vec + KM;
     constexpr int LN = 4;             // lanes per cell: a cell's rows of X and psi are fetched in one go
-    constexpr int NX = KM / LN, NQ = 24 / LN;   // a handle takes at most 24 ordinates
+    constexpr int NX = KM / LN, NQ = QMAX / LN;
+    static_assert(KM % LN == 0 && QMAX % LN == 0, "whole rows of X and of the ordinates");
     const int ln = threadIdx.x % LN;
     const auto sum4 = [](double a) {
         a += __shfl_xor_sync(0xffffffffu, a, 1);

@@ -130,6 +130,7 @@ __device__ __forceinline__ void gram_acc(double* acc, int off, const double* tA,
 // Tiles hold at most TR rows; thread t owns the columns j, j + 1 of row r of
 // such a tile, so that one load of 16 bytes a thread fetches it.
 static_assert(TR % 8 == 0 && TR * KM / 2 <= NT, "a pair of columns per thread");
+static_assert(QMAX <= KM && KM % 2 == 0 && QM % 2 == 0, "rows of the ordinates by the same pairs");
 struct Pair {
     int r, j;
     __device__ Pair() : r(threadIdx.x / (KM / 2)), j(2 * (threadIdx.x % (KM / 2))) {}

@@ -73,8 +73,8 @@ static int validate(const titus_problem_t* pb, int nz = 0) {
     if (pb->n_moments != (pb->npn + 1) * (pb->npn + 1))
         return fail(TITUS_ERR_ARG, "n_moments %d != (npn+1)^2", pb->n_moments);
     if (pb->n_ordinates < 1) return fail(TITUS_ERR_ARG, "n_ordinates < 1");
-    if (pb->n_ordinates > std::min(QM, KM))
-        return fail(TITUS_ERR_LIMIT, "n_ordinates %d > %d supported", pb->n_ordinates, std::min(QM, KM));
+    if (pb->n_ordinates > QMAX)
+        return fail(TITUS_ERR_LIMIT, "n_ordinates %d > %d supported", pb->n_ordinates, QMAX);
     if (pb->n_energies < 2) return fail(TITUS_ERR_ARG, "n_energies < 2");
     if (pb->r < 1) return fail(TITUS_ERR_ARG, "r < 1");
     if (pb->r > 2 * wide::RA)
@@ -668,5 +668,5 @@ extern "C" int titus_debug_fail_alloc(int32_t after) {
 }
 
 extern "C" int titus_max_rank(void) { return 2 * wide::RA; }
-extern "C" int titus_max_ordinates(void) { return QM < KM ? QM : KM; }
+extern "C" int titus_max_ordinates(void) { return QMAX; }
 extern "C" const char* titus_version(void) { return "titus-b200 0.1 (sm_100a, FP64)"; }

@@ -148,7 +148,7 @@ extern "C" int titus_solve_noalloc(const titus_problem_t* pb, const titus_option
     if (pb->nx < 3 || pb->ny < 3) return eo.set(TITUS_ERR_ARG, "titus_solve_noalloc: need nx, ny >= 3");
     if (pb->npn < 0 || pb->n_moments != (pb->npn + 1) * (pb->npn + 1))
         return eo.set(TITUS_ERR_ARG, "titus_solve_noalloc: n_moments != (npn+1)^2");
-    if (pb->n_ordinates < 1 || pb->n_ordinates > (QM < KM ? QM : KM))
+    if (pb->n_ordinates < 1 || pb->n_ordinates > QMAX)
         return eo.set(TITUS_ERR_LIMIT, "titus_solve_noalloc: n_ordinates outside [1, 24]");
     if (pb->r < 1 || pb->r > KM || pb->r > pb->n_moments)
         return eo.set(TITUS_ERR_LIMIT, "titus_solve_noalloc: r outside [1, min(24, n_moments)]");
