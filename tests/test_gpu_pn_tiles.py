@@ -163,3 +163,30 @@ def test_adjoint_without_entries_in_a_column_group():
     Jr.backward()
     assert abs(J - Jr.item()) <= TOL * abs(Jr.item())
     assert rel(dose, d) <= TOL and rel(grho, density.grad) <= TOL and rel(gprof, profile.grad) <= TOL
+
+
+@pytest.mark.parametrize("nx,ny,npn,ldu,fours", [(80, 71, 3, 16, 4), (61, 60, 5, 48, 2)])
+def test_small_kernel_with_several_fours(nx, ny, npn, ldu, fours):
+    """The small kernel's CTAs of several fours of cells, the last one cut: forward and adjoint."""
+    sv = solver2d(nx, ny, npn)
+    cells = (nx - 2) * (ny - 2)
+    assert cells * sum(len(v) for _, _, v in sv.ops) < 5 * 10**6     # well inside its range
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    f = 128 // ldu
+    while f > 1 and cells < 2 * sms * 4 * f:
+        f -= 1
+    assert f == fours and cells % (4 * fours)
+    with torch.no_grad():
+        ref = sweep(sv, 6, torch.tensor(sv.density).cuda(), torch.tensor(sv.bc_space).cuda())
+    u, dose, psi = SolveFirstCollisionSource(sv, max_steps=6)
+    assert rel(u, 0.5 * np.sqrt(2.0) * ref[0]) <= TOL and rel(dose, ref[1]) <= TOL and rel(psi, ref[2]) <= TOL
+    rng = np.random.default_rng(9)
+    w, t = rng.uniform(0.5, 1.5, sv.n), rng.uniform(0.0, 1.0, sv.n)
+    J, dose, grho, gprof = DoseAdjoint(sv, w, t, checkpoint_every=2, max_steps=5)
+    density = torch.tensor(sv.density).cuda().requires_grad_(True)
+    profile = torch.tensor(sv.bc_space).cuda().requires_grad_(True)
+    _, d, _ = sweep(sv, 5, density, profile)
+    Jr = (torch.from_numpy(w).cuda() * (d - torch.from_numpy(t).cuda()) ** 2).sum()
+    Jr.backward()
+    assert abs(J - Jr.item()) <= TOL * abs(Jr.item())
+    assert rel(dose, d) <= TOL and rel(grho, density.grad) <= TOL and rel(gprof, profile.grad) <= TOL
