@@ -89,11 +89,10 @@ BATCHED = dict(name="pencil_beams256_phantom_128x128_P21_cap60_bug", Nx=129, r=6
 BATCHED_SAMPLE_ITERS = 600
 FIXTURE = os.path.join(ROOT, "tests", "golden", "phantom200_P29_bug200.npz")
 RANKS_FIXTURE = os.path.join(ROOT, "tests", "golden", "phantom200_P29_bug_ranks.npz")
-# DRAM bytes (read + write) per energy step of each kernel on its workload, from
-# one ncu capture of the first energy steps (profiles/); the per-launch figure
-# scales it to the launch's energy steps.
-DRAM_BYTES_PER_STEP_NCU = {"fixed": (5.010176e6 + 0.218112e6) / 20,
-                           "bug": (77.263616e6 + 193.732352e6) / 20, "parallel": None}
+# DRAM bytes (read + write) per energy step of each kernel on its workload, from an
+# ncu capture; the per-launch figure scales it to the launch's energy steps. None: the
+# present kernel has no capture (those in profiles/ are of its forms with 256 threads).
+DRAM_BYTES_PER_STEP_NCU = {"fixed": None, "bug": None, "parallel": None}
 
 
 def algorithmic_bytes_per_step(n, r, q, w=8):
@@ -846,7 +845,8 @@ def run_gpu(args, w, rank, world, local_rank):
                              "frac": info["achieved"] / peak,
                              "traffic": (info["traffic_step"] * info["steps_per_solve"]
                                          if info["traffic_step"] else None),
-                             "traffic_note": "ncu capture of the first energy steps scaled to the launch's steps",
+                             "traffic_note": ("ncu capture of the first energy steps scaled to the launch's steps"
+                                              if info["traffic_step"] else "no capture of the present kernel"),
                              "peak_kind": info["peak_kind"], "algorithmic_bytes_per_launch": info["alg_bytes"]},
                 "cpu_baseline": None,
                 "clocks": info["clocks"],

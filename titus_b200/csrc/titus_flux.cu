@@ -37,7 +37,8 @@ constexpr int kFluxThreads = 128;
 // the unrolling of the row loop. Without rows ahead the loop waited for one load
 // from memory a row (468 us at 2048 x 2048 x 16, 65 % of the stalls); measured
 // there with (cells, ahead, unroll): (2,1,1) 323, (2,3,2) 293, (4,1,1) 310,
-// (4,2,1) 317, (4,3,1) 287, (4,3,2) 271, (4,4,2) 321 us; at 1024 x 1024 79 us.
+// (4,2,1) 317, (4,3,1) 287, (4,3,2) 271, (4,4,2) 321 us of kernel; at 1024 x 1024 80 us.
+// A call from Python among others takes 281 to 296 us at 2048 x 2048.
 constexpr int kCells = 4, kAhead = 3, kUnroll = 2;
 
 // Rows a thread walks: 32 where that leaves 150 000 threads, else as many fewer

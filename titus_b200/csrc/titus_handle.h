@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "../../include/titus.h"
@@ -71,11 +72,12 @@ int wide_solve_batched(titus_solver* s, int method, const titus_options_t* opt, 
 // Default team of a solve. Solves on the default stream follow one another, so each may
 // take `alone` CTAs, up to the whole chip. A caller's own stream is how a program runs
 // several handles side by side: there a team keeps to `beside` CTAs, since with one CTA
-// per SM a larger team would make the others wait. Microseconds per solve and step,
-// teams of `alone` and of `beside` CTAs: fixed rank 100 x 100, r = 20: one solve 592 and
-// 754, four side by side 590 and 188; RK4 there 578 and 808, four 575 and 206; BUG
-// 200 x 200, P29: one 834 and 898, two 824 and 505; BUG 100 x 100, P21: one 834 and 841,
-// two 835 and 435; parallel 128 x 128, P21: one 500 and 494, two 502 and 252.
+// per SM a larger team would make the others wait. Microseconds per solve and step over
+// the first 40 to 200 steps of a solve, teams of `alone` and of `beside` CTAs: fixed rank
+// 100 x 100, r = 20: one solve 592 and 754, four side by side 590 and 188; RK4 there 578
+// and 808, four 575 and 206; BUG 200 x 200, P29: one 834 and 898, two 824 and 505; BUG
+// 100 x 100, P21: one 834 and 841, two 835 and 435; parallel 128 x 128, P21: one 500 and
+// 494, two 502 and 252.
 inline int default_team(int alone, int beside, cudaStream_t stream) {
     const bool own = stream != nullptr && stream != cudaStreamLegacy;
     return own ? std::min(alone, beside) : alone;

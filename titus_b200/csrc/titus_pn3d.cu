@@ -29,7 +29,7 @@ namespace {
 
 constexpr int P3_NT = 256;
 constexpr int P3_NOP = 6;
-// Largest moment count taken (P64).
+// Largest moment count taken: P64. It is the interface's, not the kernels' (titus_pn_full.cu).
 constexpr int P3_MAX_MOMENTS = 4266;
 
 // 4 x 2 x 8 cells, 56 operator tiles a stage, two CTAs a SM: as many tiles as fit beside

@@ -27,7 +27,9 @@ using titus_pn::PtArgs;
 namespace {
 
 constexpr int PN_NT = 256;    // threads per CTA of the cell-wise kernels
-// Largest moment counts taken (P59 forward, P39 adjoint).
+// Largest moment counts taken: P59 forward, P39 adjoint. They are the interface's; the
+// kernels need no more shared memory for more moments (pt_patches leaves the small
+// kernel where its images would not fit), only longer tables.
 constexpr int PN_MAX_MOMENTS = 3632, ADJ_MAX_MOMENTS = 1600;
 
 // 8 x 8 cells, 96 operator tiles a stage, two CTAs a SM: as many tiles as fit beside

@@ -271,7 +271,7 @@ __device__ __forceinline__ bool gram_finish(TcCtx& t) {
 }
 
 // Read the accumulators back: for every valid (m < mw, n < nw) call
-// out(m, n, value) with the FP32 sum. Warps w and w + 4 share TMEM lane
+// out(m, n, value) with the FP32 sum. Warps w, w + 4, w + 8, .. share TMEM lane
 // quadrant w % 4 and split the 16-column groups between them.
 template <int NTH, class Out>
 __device__ void gram_read(const TcCtx& t, const GramShape& g, Out out) {

@@ -465,7 +465,7 @@ static __device__ __noinline__ int w_svd_complete(double* At, double* Vt, int ld
                 }
                 int found = -1;
                 if (cand < nrows) {
-                    // next row with norm > 1e-6, eight candidates at a time (one per warp)
+                    // next row with norm > 1e-6, a candidate per warp at a time
                     while (cand < nrows && found < 0) {
                         const int c = cand + warp;
                         double sq = 0.0;
